@@ -48,6 +48,51 @@ EDGE_D float sel3(const float v[3], int a) { return a == 0 ? v[0] : (a == 1 ? v[
 EDGE_D int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 // ---------------------------------------------------------------------------
+// Two floats in one 64-bit register, for the packed FP32 instructions of
+// sm_100 (fma.rn.f32x2 and mul.rn.f32x2).  They have the FP32 peak of the
+// scalar ones (67 against 65 TFLOP/s, independent chains) but take half the
+// issue slots, and an operand that is one float in both halves (`both`) needs
+// no instruction of its own.  Each half rounds as the scalar instruction does.
+// A multiply-add whose three operands are different registers is bound by the
+// register ports: measured 1.84 cycles scalar, 2.71 cycles per pair.
+// ---------------------------------------------------------------------------
+struct f2 {
+    unsigned long long v;
+};
+EDGE_D f2 pair(float lo, float hi) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+EDGE_D f2 both(float a) { return pair(a, a); }
+EDGE_D float lo(f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return x;
+}
+EDGE_D float hi(f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return y;
+}
+EDGE_D f2 fma2(f2 a, f2 b, f2 c) {
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return d;
+}
+EDGE_D f2 mul2(f2 a, f2 b) {
+    f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+    return d;
+}
+// a0 b0 + a1 b1 + a2 b2 with the roundings of the scalar expression as nvcc
+// contracts it (the products of the inner sum: the first is fused)
+EDGE_D f2 dot3(f2 a0, f2 b0, f2 a1, f2 b1, f2 a2, f2 b2) { return fma2(a2, b2, fma2(a0, b0, mul2(a1, b1))); }
+EDGE_D float dot3(float a0, float b0, float a1, float b1, float a2, float b2) {
+    return __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1)));
+}
+
+// ---------------------------------------------------------------------------
 // quadratic B-spline (taichi_utils.py:230-251) evaluated separably on the three
 // non-zero taps of each axis
 // ---------------------------------------------------------------------------
@@ -68,73 +113,119 @@ EDGE_D float dN2(float x) {
 
 // One axis of interp_2 / interp_grad_2 (taichi_utils.py:254-319): the clamped
 // grid coordinate, the first of the three taps that carry weight (the 4th tap
-// of the reference's -1..2 loop is always zero) and their weights.
-struct Axis3 {
+// of the reference's -1..2 loop is always zero) and their weights; with GRAD
+// each weight is paired with its derivative, w[t] = (N2, N2').
+template <bool GRAD>
+struct Axis3;
+template <>
+struct Axis3<false> {
     int base;
     float w[3];
-    float dw[3];
 };
+template <>
+struct Axis3<true> {
+    int base;
+    f2 w[3];
+};
+EDGE_D void set_tap(float& w, float v, float) { w = v; }
+EDGE_D void set_tap(f2& w, float v, float d) { w = pair(v, d); }
+
 template <bool GRAD>
-EDGE_D Axis3 bspline_axis(float u, float hi) {
-    Axis3 a;
-    float s = fmaxf(1.0f, fminf(u, hi));
-    float iu = floorf(s);
-    const float bf = (s - iu < 0.5f) ? iu - 1.0f : iu;  // the first tap, an integer held exactly
-    float x0 = s - bf;
+EDGE_D Axis3<GRAD> bspline_axis(float u, float hi_) {
+    Axis3<GRAD> a;
+    const float s = fmaxf(1.0f, fminf(u, hi_));
+    // the first tap, an integer held exactly; s >= 1, so s - 0.5 is exact
+    const float bf = floorf(s - 0.5f);
+    const float x0 = s - bf;
     a.base = (int)bf;
-    // x0 lies in [0.5, 1.5) (exactly: s - b is exact), so the branches of
-    // N2 / dN2 at x0, x0 - 1 and x0 - 2 are known: the same operations as the
+    // x0 lies in [0.5, 1.5) (exactly: s - bf is exact), so the branches of
+    // N2 / dN2 at x0, x0 - 1 and x0 - 2 are known: the same values as the
     // general functions, without their compares.  The third tap's zero
     // branch (|x0 - 2| = 1.5, i.e. x0 = 0.5) needs no select either: there
-    // t2 = 0 and 2 a2 - 3 = 0, so the polynomial gives the same zero; and
-    // |x1| |x1| = x1 x1, sign(x1) * (-2 |x1|) = -2 x1 exactly.
-    const float x1 = x0 - 1.0f, x2 = x0 - 2.0f;  // x1 in [-0.5, 0.5), x2 in [-1.5, -0.5)
-    const float t0 = 1.5f - x0, a2 = -x2, t2 = 1.5f - a2;
-    a.w[0] = 0.5f * (t0 * t0);
-    a.w[1] = 0.75f - x1 * x1;
-    a.w[2] = 0.5f * (t2 * t2);
-    if (GRAD) {
-        a.dw[0] = 0.5f * (2.0f * x0 - 3.0f);
-        a.dw[1] = -2.0f * x1;
-        a.dw[2] = -(0.5f * (2.0f * a2 - 3.0f));
-    }
+    // t2 = x0 - 0.5 = 0.  Every difference below is exact, so the first and
+    // third derivatives (2 |x| - 3) / 2 are x0 - 1.5 and x0 - 0.5.
+    const float x1 = x0 - 1.0f, t0 = 1.5f - x0, t2 = x0 - 0.5f;
+    set_tap(a.w[0], (0.5f * t0) * t0, x0 - 1.5f);
+    set_tap(a.w[1], 0.75f - x1 * x1, -2.0f * x1);
+    set_tap(a.w[2], (0.5f * t2) * t2, t2);
     return a;
 }
 
-// 27-tap separable contraction of one scalar field; g receives the gradient
-// (already multiplied by 1/dx) when GRAD.
-template <bool GRAD>
-EDGE_D float bspline_sum(const float* __restrict__ f, int n1, int n2, const Axis3& X, const Axis3& Y,
-                         const Axis3& Z, float inv_dx, float* g) {
-    float v = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
+// Row pointer of tap row (i, j): one 32-bit byte offset per sample added to
+// the row's uniform address, so that a row costs one add and its taps are
+// immediate offsets.  BIG: grids whose faces may pass 4 GB per component.
+template <bool BIG>
+EDGE_D const float* tap_row(const float* f, int e, int i, int j, int n1, int n2) {
+    if (BIG) return f + e + (i * n1 + j) * n2;
+    return reinterpret_cast<const float*>(reinterpret_cast<const char*>(f + (i * n1 + j) * n2) + 4u * (unsigned)e);
+}
+
+// 27-tap separable contraction of one scalar field, z then y then x, value and
+// gradient (already multiplied by 1/dx).  (weight, derivative) pairs against
+// taps in both halves give each row's value and z derivative in one packed
+// multiply-add per tap, and the y and x sums carry the same pair.  The kernels
+// this runs in are bound by FP32 register ports and issue slots: 690 thread
+// instructions per three-component sample with scalar multiply-adds and 64-bit
+// row addresses, 515 in this form (RK4 with Jacobian of 128^3 cells, 12
+// samples each: 0.611 -> 0.508 ms, the same bits).
+template <bool BIG>
+EDGE_D float bspline_sum(const float* __restrict__ f, int n1, int n2, const Axis3<true>& X, const Axis3<true>& Y,
+                         const Axis3<true>& Z, float inv_dx, float* g) {
+    f2 vz = both(0.0f);  // (value, z derivative)
+    float gx = 0.0f, gy = 0.0f;
+    const int e = idx3(X.base, Y.base, Z.base, n1, n2);
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        float cv = 0.0f, cy = 0.0f, cz = 0.0f;
+        f2 c = both(0.0f);
+        float cy = 0.0f;
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            const float* row = f + idx3(X.base + i, Y.base + j, Z.base, n1, n2);
-            float q0 = __ldg(row), q1 = __ldg(row + 1), q2 = __ldg(row + 2);
-            float a = Z.w[0] * q0 + Z.w[1] * q1 + Z.w[2] * q2;
-            cv += Y.w[j] * a;
-            if (GRAD) {
-                float dz = Z.dw[0] * q0 + Z.dw[1] * q1 + Z.dw[2] * q2;
-                cy += Y.dw[j] * a;
-                cz += Y.w[j] * dz;
-            }
+            const float* row = tap_row<BIG>(f, e, i, j, n1, n2);
+            const f2 a = dot3(Z.w[0], both(__ldg(row)), Z.w[1], both(__ldg(row + 1)), Z.w[2], both(__ldg(row + 2)));
+            c = fma2(both(lo(Y.w[j])), a, c);
+            cy = __fmaf_rn(hi(Y.w[j]), lo(a), cy);
         }
-        v += X.w[i] * cv;
-        if (GRAD) {
-            gx += X.dw[i] * cv;
-            gy += X.w[i] * cy;
-            gz += X.w[i] * cz;
+        vz = fma2(both(lo(X.w[i])), c, vz);
+        gx = __fmaf_rn(hi(X.w[i]), lo(c), gx);
+        gy = __fmaf_rn(lo(X.w[i]), cy, gy);
+    }
+    g[0] = gx * inv_dx;
+    g[1] = gy * inv_dx;
+    g[2] = hi(vz) * inv_dx;
+    return lo(vz);
+}
+
+// The value alone: rows of equal j are paired over i = 0, 1 and the first two
+// rows of i = 2 over j, so that the 27 row products take 15 instructions.  All
+// 27 taps are loaded before the first is used: the kernels that take one
+// sample per thread wait for their gathers (velocity pullback at 256x128x128
+// 344 us row by row, 322 us so, 343 us with the scalar sampler).
+template <bool BIG>
+EDGE_D float bspline_sum(const float* __restrict__ f, int n1, int n2, const Axis3<false>& X, const Axis3<false>& Y,
+                         const Axis3<false>& Z, float, float*) {
+    const int e = idx3(X.base, Y.base, Z.base, n1, n2);
+    float q[3][3][3];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const float* row = tap_row<BIG>(f, e, i, j, n1, n2);
+#pragma unroll
+            for (int k = 0; k < 3; k++) q[i][j][k] = __ldg(row + k);
         }
-    }
-    if (GRAD) {
-        g[0] = gx * inv_dx;
-        g[1] = gy * inv_dx;
-        g[2] = gz * inv_dx;
-    }
-    return v;
+    auto rows = [&](const float (&a)[3], const float (&b)[3]) {
+        return dot3(both(Z.w[0]), pair(a[0], b[0]), both(Z.w[1]), pair(a[1], b[1]), both(Z.w[2]), pair(a[2], b[2]));
+    };
+    f2 c01 = both(0.0f);
+#pragma unroll
+    for (int j = 0; j < 3; j++) c01 = fma2(both(Y.w[j]), rows(q[0][j], q[1][j]), c01);
+    const f2 a2 = rows(q[2][0], q[2][1]);
+    float c2 = __fmaf_rn(Y.w[0], lo(a2), 0.0f);
+    c2 = __fmaf_rn(Y.w[1], hi(a2), c2);
+    c2 = __fmaf_rn(Y.w[2], dot3(Z.w[0], q[2][2][0], Z.w[1], q[2][2][1], Z.w[2], q[2][2][2]), c2);
+    float v = __fmaf_rn(X.w[0], lo(c01), 0.0f);
+    v = __fmaf_rn(X.w[1], hi(c01), v);
+    return __fmaf_rn(X.w[2], c2, v);
 }
 
 // MAC velocity field + the clamp bounds of its three staggered components.
@@ -162,19 +253,19 @@ static inline Mac make_mac(const float* ux, const float* uy, const float* uz, in
 
 // interp_u_MAC / interp_u_MAC_grad (taichi_utils.py:322-341).  G rows are the
 // gradients of u_x, u_y, u_z.
-template <bool GRAD>
+template <bool GRAD, bool BIG = false>
 EDGE_D void mac_sample(const Mac& m, const float p[3], float v[3], float G[3][3]) {
     float q[3] = {over_dx(p[0], m.dx, m.inv_dx, m.pow2), over_dx(p[1], m.dx, m.inv_dx, m.pow2),
                   over_dx(p[2], m.dx, m.inv_dx, m.pow2)};
-    Axis3 A0[3], A5[3];
+    Axis3<GRAD> A0[3], A5[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         A0[d] = bspline_axis<GRAD>(q[d], m.hi0[d]);
         A5[d] = bspline_axis<GRAD>(q[d] - 0.5f, m.hi5[d]);
     }
-    v[0] = bspline_sum<GRAD>(m.u[0], m.ny, m.nz, A0[0], A5[1], A5[2], m.inv_dx, GRAD ? G[0] : nullptr);
-    v[1] = bspline_sum<GRAD>(m.u[1], m.ny + 1, m.nz, A5[0], A0[1], A5[2], m.inv_dx, GRAD ? G[1] : nullptr);
-    v[2] = bspline_sum<GRAD>(m.u[2], m.ny, m.nz + 1, A5[0], A5[1], A0[2], m.inv_dx, GRAD ? G[2] : nullptr);
+    v[0] = bspline_sum<BIG>(m.u[0], m.ny, m.nz, A0[0], A5[1], A5[2], m.inv_dx, GRAD ? G[0] : nullptr);
+    v[1] = bspline_sum<BIG>(m.u[1], m.ny + 1, m.nz, A5[0], A0[1], A5[2], m.inv_dx, GRAD ? G[1] : nullptr);
+    v[2] = bspline_sum<BIG>(m.u[2], m.ny, m.nz + 1, A5[0], A5[1], A0[2], m.inv_dx, GRAD ? G[2] : nullptr);
 }
 
 // Component a of interp_u_MAC alone (mac_sample's arithmetic for that
@@ -183,7 +274,7 @@ EDGE_D void mac_sample(const Mac& m, const float p[3], float v[3], float G[3][3]
 EDGE_D float mac_sample_comp(const Mac& m, const float p[3], int a) {
     float q[3] = {over_dx(p[0], m.dx, m.inv_dx, m.pow2), over_dx(p[1], m.dx, m.inv_dx, m.pow2),
                   over_dx(p[2], m.dx, m.inv_dx, m.pow2)};
-    Axis3 A[3];
+    Axis3<false> A[3];
 #pragma unroll
     for (int d = 0; d < 3; d++)
         A[d] = d == a ? bspline_axis<false>(q[d], m.hi0[d]) : bspline_axis<false>(q[d] - 0.5f, m.hi5[d]);
@@ -697,54 +788,63 @@ EDGE_D void rk4_pos(const Mac& mac, float psi[3], float dt) {
 
 // RK4 of a point with NC Jacobian columns C[a] (dC/dt = grad u . C).  The
 // four stages run as a loop (not unrolled): one copy of the 81-tap sampler
-// keeps the kernels inside the instruction cache.
+// keeps the kernels inside the instruction cache.  Columns 0 and 1 are
+// advanced as pairs.
 template <int NC>
 EDGE_D void rk4_jac(const Mac& mac, float psi[3], float C[NC][3], float dt) {
-    float u[3], G[3][3], q[3], Cs[NC][3], d[NC][3], su[3] = {0.0f, 0.0f, 0.0f}, sd[NC][3];
-    float h = 0.5f * dt;
+    static_assert(NC == 1 || NC == 3, "one column, or all three");
+    constexpr int L = NC - 1;  // the column advanced on its own
+    float u[3], G[3][3], q[3], su[3], s1[3], S1[3];
+    f2 C2[3], s2[3], S2[3];
+    const float h = 0.5f * dt;
 #pragma unroll
-    for (int a = 0; a < NC; a++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) sd[a][c] = 0.0f;
-#pragma unroll
-    for (int c = 0; c < 3; c++) q[c] = psi[c];
-#pragma unroll
-    for (int a = 0; a < NC; a++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) Cs[a][c] = C[a][c];
+    for (int c = 0; c < 3; c++) {
+        q[c] = psi[c];
+        su[c] = 0.0f;  // the RK4 sums, started at zero: 0 + 1 * u is u exactly
+        s1[c] = C[L][c];
+        S1[c] = 0.0f;
+        if (NC == 3) {
+            C2[c] = s2[c] = pair(C[0][c], C[NC - 2][c]);
+            S2[c] = both(0.0f);
+        }
+    }
 #pragma unroll 1
     for (int stage = 0; stage < 4; stage++) {
         mac_sample<true>(mac, q, u, G);
-        // derivative of the columns at this stage
-#pragma unroll
-        for (int a = 0; a < NC; a++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) d[a][r] = G[r][0] * Cs[a][0] + G[r][1] * Cs[a][1] + G[r][2] * Cs[a][2];
-        // the RK4 sums, started at zero: 0 + 1 * u is u exactly
         const float wt = (stage == 0 || stage == 3) ? 1.0f : 2.0f;
+        const float hh = stage < 2 ? h : dt;
+        // derivative of the columns at this stage, their sums and the next
+        // stage's point
+        float d1[3];
+        f2 d2[3];
 #pragma unroll
-        for (int c = 0; c < 3; c++) su[c] = su[c] + wt * u[c];
+        for (int r = 0; r < 3; r++) {
+            d1[r] = dot3(G[r][0], s1[0], G[r][1], s1[1], G[r][2], s1[2]);
+            if (NC == 3) d2[r] = dot3(both(G[r][0]), s2[0], both(G[r][1]), s2[1], both(G[r][2]), s2[2]);
+        }
 #pragma unroll
-        for (int a = 0; a < NC; a++)
-#pragma unroll
-            for (int c = 0; c < 3; c++) sd[a][c] = sd[a][c] + wt * d[a][c];
-        if (stage < 3) {
-            const float hh = stage < 2 ? h : dt;
-#pragma unroll
-            for (int c = 0; c < 3; c++) q[c] = psi[c] + hh * u[c];
-#pragma unroll
-            for (int a = 0; a < NC; a++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) Cs[a][c] = C[a][c] + hh * d[a][c];
+        for (int c = 0; c < 3; c++) {
+            su[c] = __fmaf_rn(wt, u[c], su[c]);
+            q[c] = __fmaf_rn(hh, u[c], psi[c]);
+            S1[c] = __fmaf_rn(wt, d1[c], S1[c]);
+            s1[c] = __fmaf_rn(hh, d1[c], C[L][c]);
+            if (NC == 3) {
+                S2[c] = fma2(both(wt), d2[c], S2[c]);
+                s2[c] = fma2(both(hh), d2[c], C2[c]);
+            }
         }
     }
-    float w6 = dt * 1.0f / 6.0f;
+    const float w6 = dt * 1.0f / 6.0f;
 #pragma unroll
-    for (int c = 0; c < 3; c++) psi[c] = psi[c] + w6 * su[c];
-#pragma unroll
-    for (int a = 0; a < NC; a++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) C[a][c] = C[a][c] + w6 * sd[a][c];
+    for (int c = 0; c < 3; c++) {
+        psi[c] = __fmaf_rn(w6, su[c], psi[c]);
+        if (NC == 3) {
+            const f2 t = fma2(both(w6), S2[c], C2[c]);
+            C[0][c] = lo(t);
+            C[NC - 2][c] = hi(t);
+        }
+        C[L][c] = __fmaf_rn(w6, S1[c], C[L][c]);
+    }
 }
 
 EDGE_D void cell_pos(int i, int j, int k, float dx, float X[3]) {

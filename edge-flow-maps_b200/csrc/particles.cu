@@ -29,8 +29,8 @@ __global__ void k_lp_acc(Mac mac_, const float* __restrict__ vel, const float* _
     if (e < num) {
         float kk = 1.0f / St;
         float p[3] = {pos[3 * e], pos[3 * e + 1], pos[3 * e + 2]};
-        float v[3], G[3][3];
-        mac_sample<true>(mac, p, v, G);
+        float v[3];
+        mac_sample<false, true>(mac, p, v, nullptr);
         a[1] += gravity;
         for (int c = 0; c < 3; c++) a[c] -= kk * (vel[3 * e + c] - v[c]);
         for (int c = 0; c < 3; c++) a[c] /= (1.0f + kk * dt);
@@ -62,8 +62,8 @@ __global__ void k_lp_vel_diff(Mac mac_, const float* __restrict__ vel, float* vd
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= num) return;
     float p[3] = {pos[3 * e], pos[3 * e + 1], pos[3 * e + 2]};
-    float v[3], G[3][3];
-    mac_sample<true>(mac, p, v, G);
+    float v[3];
+    mac_sample<false, true>(mac, p, v, nullptr);
     for (int c = 0; c < 3; c++) vdiff[3 * e + c] = kk * (vel[3 * e + c] - v[c]);
 }
 
