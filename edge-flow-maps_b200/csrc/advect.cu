@@ -560,29 +560,126 @@ __global__ void k_coef_p(MapP m, float4* __restrict__ g) {
     g[(size_t)7 * n + e] = make_float4(o[3][0], o[3][1], o[3][2], 0.f);
 }
 
-// face map on the packed layout, one launch per face axis A: the map at the
-// face and the derivative along A (only that gradient column is evaluated)
-// (register caps: ED4 / EDGE 128 registers, 4 CTAs per SM; ED8 102, 5 CTAs
-// per SM; both measured faster than the uncapped builds)
-template <int V, int A, bool P2>
-__global__ void __launch_bounds__(128, V == HV_FULL ? 5 : 4) k_face_map_p(MapP m_, float* fp, float* fc) {
-    const MapP m = with_pow2<P2>(m_);
-    const int n1 = m.ny + (A == 1), n2 = m.nz + (A == 2);
-    const long long nf = (long long)(m.nx + (A == 0)) * n1 * n2;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nf) return;
-    const unsigned u = (unsigned)t;  // one face grid: fits 32 bits
-    const int e = (int)u;
-    const int k = (int)(u % (unsigned)n2);
-    const unsigned r = u / (unsigned)n2;
-    const int j = (int)(r % (unsigned)n1), i = (int)(r / (unsigned)n1);
-    float X[3], val[3], G[3][3];
-    face_pos(A, i, j, k, m.dx, X);
-    hermite3p<V, true, A>(m, X, val, G);
+// Face map on the packed layout.  A face centre lies on the line between the
+// centres of the two cells it separates, so its Hermite coordinate across its
+// own axis is the only one with a fractional part: in the other two axes the
+// f basis is exactly 1 at the base corner and 0 at the next and the g basis
+// exactly 0, and of the 64 coefficients of the 8 corners four remain, psi and
+// its derivative along the axis at two cells.  The sum of those is the full
+// contraction's value bit for bit on a finite map (every other term adds 0).
+// The fractional part is taken from the coordinate as the full evaluation
+// forms it; where rounding leaves it non-zero (spacings that are no power of
+// two, and the clamped last cell of a short axis) the face is left to
+// k_face_map_rest.  Bound by memory: 4 planes in, 24 bytes per face out.
+// 256x128x128: 818 us for one 64-coefficient launch per axis, 111 us so (the
+// copy bandwidth allows 90); 192x96x96, where a quarter of the faces is left
+// over: 363 and 218 us.
+struct Face3 {
+    const float* p[3];
+    // select with constant indices only: a run-time index into a kernel
+    // parameter array makes the compiler copy the parameter to local memory
+    EDGE_D const float* at(int a) const { return a == 0 ? p[0] : (a == 1 ? p[1] : p[2]); }
+};
+struct Face3W {
+    float* p[3];
+    EDGE_D float* at(int a) const { return a == 0 ? p[0] : (a == 1 ? p[1] : p[2]); }
+};
+
+// Hermite coordinate of axis d's cell centre i as hermite3p forms it: its base
+// cell, and whether it has no fractional part
+struct Centre {
+    int c;
+    bool exact;
+};
+EDGE_D Centre centre_of(const MapP& m, int i, float hi) {
+    const float u = over_dx(((float)i + 0.5f) * m.dx, m.dx, m.inv_dx, m.pow2) - 0.5f;
+    const float s = fmaxf(1.0f, fminf(u, hi)), b = floorf(s);
+    return Centre{(int)b, s == b};
+}
+
+// the face between cells ea and eb, `plane` the derivative along its axis
+EDGE_D void face_line(const MapP& m, const HAxis& H, int plane, int ea, int eb, float* fp, float* fc) {
+    const float4 P0 = ldp(m, 0, ea), D0 = ldp(m, plane, ea), P1 = ldp(m, 0, eb), D1 = ldp(m, plane, eb);
+    const float inv = 1.0f / m.dx;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-        fp[3 * e + c] = val[c];
-        fc[3 * e + c] = G[c][A];
+        const float a = c4(P0, c), b = c4(P1, c);
+        const float ga = m.pow2 ? c4(D0, c) : c4(D0, c) * m.dx, gb = m.pow2 ? c4(D1, c) : c4(D1, c) * m.dx;
+        fp[c] = __fadd_rn(__fmaf_rn(H.f[0], a, __fmul_rn(H.g[0], ga)), __fmaf_rn(H.f[1], b, __fmul_rn(H.g[1], gb)));
+        fc[c] = __fadd_rn(__fmaf_rn(H.df[0], a, __fmul_rn(H.dg[0], ga)),
+                          __fmaf_rn(H.df[1], b, __fmul_rn(H.dg[1], gb))) * inv;
+    }
+}
+
+// one thread per cell: its three low faces (so that psi is read once for the
+// three axes) and, in the last cell of an axis, the high face too
+template <bool P2>
+__global__ void __launch_bounds__(128) k_face_line_p(MapP m_, Face3W fp, Face3W fc) {
+    const MapP m = with_pow2<P2>(m_);
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= m.n) return;
+    const int ix[3] = {e / (m.ny * m.nz), (e / m.nz) % m.ny, e % m.nz}, dim[3] = {m.nx, m.ny, m.nz};
+    const int st[3] = {m.ny * m.nz, m.nz, 1};
+    Centre C[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) C[d] = centre_of(m, ix[d], m.hi[d]);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
+        if (!C[b].exact || !C[c].exact) continue;
+        const int row = C[b].c * st[b] + C[c].c * st[c];
+        const int n1 = m.ny + (a == 1), n2 = m.nz + (a == 2);
+        const int highs = ix[a] == dim[a] - 1 ? 2 : 1;
+        for (int h = 0; h < highs; h++) {
+            HAxis H = haxis(over_dx((float)(ix[a] + h) * m.dx, m.dx, m.inv_dx, m.pow2) - 0.5f, m.hi[a], dim[a]);
+            if (m.pow2) {
+                H.g[0] *= m.dx; H.g[1] *= m.dx;
+                H.dg[0] *= m.dx; H.dg[1] *= m.dx;
+            }
+            float v[3], g[3];
+            face_line(m, H, 1 + a, row + H.c0 * st[a], row + H.cp * st[a], v, g);
+            const int f = idx3(ix[0] + (a == 0 ? h : 0), ix[1] + (a == 1 ? h : 0), ix[2] + (a == 2 ? h : 0), n1, n2);
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                fp.p[a][3 * f + q] = v[q];
+                fc.p[a][3 * f + q] = g[q];
+            }
+        }
+    }
+}
+
+// The faces k_face_line_p leaves: each block looks over `chunk` faces,
+// collects those in shared memory and evaluates them with full warps (they
+// are single k in nearly every warp when the spacing is no power of two:
+// about a quarter of all faces).
+constexpr int kRestFaces = 1024;  // most faces of a block
+template <int V, bool P2>
+__global__ void __launch_bounds__(128) k_face_map_rest(MapP m_, Face3W fp, Face3W fc, int chunk) {
+    const MapP m = with_pow2<P2>(m_);
+    __shared__ int list[kRestFaces];
+    __shared__ int count;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    const long long base = (long long)blockIdx.x * chunk, nf = n_faces(m.nx, m.ny, m.nz);
+    for (int t = threadIdx.x; t < chunk && base + t < nf; t += blockDim.x) {
+        const FaceIdx f = face_decompose(base + t, m.nx, m.ny, m.nz);
+        const bool line = (f.axis == 0 || centre_of(m, f.i, m.hi[0]).exact) &&
+                          (f.axis == 1 || centre_of(m, f.j, m.hi[1]).exact) &&
+                          (f.axis == 2 || centre_of(m, f.k, m.hi[2]).exact);
+        if (!line) list[atomicAdd(&count, 1)] = t;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < count; q += blockDim.x) {
+        const FaceIdx f = face_decompose(base + list[q], m.nx, m.ny, m.nz);
+        float X[3], val[3], G[3][3];
+        face_pos(f.axis, f.i, f.j, f.k, m.dx, X);
+        hermite3p<V, true>(m, X, val, G);
+        float *p = fp.at(f.axis) + 3 * f.e, *g = fc.at(f.axis) + 3 * f.e;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            p[c] = val[c];
+            g[c] = sel3(G[c], f.axis);
+        }
     }
 }
 
@@ -790,13 +887,6 @@ __global__ void __launch_bounds__(128) k_advect_sl(Mac mac_, float dt, float* ox
     float* o = f.axis == 0 ? ox : (f.axis == 1 ? oy : oz);
     o[f.e] = mac_sample_comp(mac, q, f.axis);
 }
-
-struct Face3 {
-    const float* p[3];
-    // select with constant indices only: a run-time index into a kernel
-    // parameter array makes the compiler copy the parameter to local memory
-    EDGE_D const float* at(int a) const { return a == 0 ? p[0] : (a == 1 ? p[1] : p[2]); }
-};
 
 // map_u / map_u_psi pullback with fused BFECC arithmetic (edge_pullback_u)
 template <bool P2>
@@ -1381,39 +1471,29 @@ int edge_face_map_packed(int variant, int nx, int ny, int nz, float dx, const fl
         return EDGE_EINVAL;
     if (!al16(packed)) return EDGE_EALIGN;
     MapP m = make_mapp(packed, nx, ny, nz, dx);
-    const int gx = grid_for((long long)(nx + 1) * ny * nz, 128), gy = grid_for((long long)nx * (ny + 1) * nz, 128),
-              gz = grid_for((long long)nx * ny * (nz + 1), 128);
+    const Face3W fp{{fpsix, fpsiy, fpsiz}}, fc{{fcolx, fcoly, fcolz}};
     cudaStream_t st = S(stream);
+    const int g = grid_for(m.n, 128);
+    if (m.pow2) k_face_line_p<true><<<g, 128, 0, st>>>(m, fp, fc);
+    else k_face_line_p<false><<<g, 128, 0, st>>>(m, fp, fc);
+    // with a power-of-two spacing only the last cell centre of an axis can be
+    // off its cell: there the clamp bound n-2-1e-6 may be below n-2 in float32
+    auto whole = [](float x) { return x == floorf(x); };
+    if (m.pow2 && whole(m.hi[0]) && whole(m.hi[1]) && whole(m.hi[2])) return launch_status();
+    // 16 blocks per SM where the grid has the faces for it: a block's collected
+    // faces take one or two rounds of its threads
+    const long long nf = n_faces(nx, ny, nz);
+    const int chunk = (int)std::min<long long>(kRestFaces, nf / (148 * 16) / 128 * 128 + 128);
+    const int r = (int)((nf + chunk - 1) / chunk);
     if (variant == HV_FD) {
-        if (m.pow2) {
-            k_face_map_p<HV_FD_P, 0, true><<<gx, 128, 0, st>>>(m, fpsix, fcolx);
-            k_face_map_p<HV_FD_P, 1, true><<<gy, 128, 0, st>>>(m, fpsiy, fcoly);
-            k_face_map_p<HV_FD_P, 2, true><<<gz, 128, 0, st>>>(m, fpsiz, fcolz);
-        } else {
-            k_face_map_p<HV_FD_P, 0, false><<<gx, 128, 0, st>>>(m, fpsix, fcolx);
-            k_face_map_p<HV_FD_P, 1, false><<<gy, 128, 0, st>>>(m, fpsiy, fcoly);
-            k_face_map_p<HV_FD_P, 2, false><<<gz, 128, 0, st>>>(m, fpsiz, fcolz);
-        }
+        if (m.pow2) k_face_map_rest<HV_FD_P, true><<<r, 128, 0, st>>>(m, fp, fc, chunk);
+        else k_face_map_rest<HV_FD_P, false><<<r, 128, 0, st>>>(m, fp, fc, chunk);
     } else if (variant == HV_GARM) {
-        if (m.pow2) {
-            k_face_map_p<HV_GARM_P, 0, true><<<gx, 128, 0, st>>>(m, fpsix, fcolx);
-            k_face_map_p<HV_GARM_P, 1, true><<<gy, 128, 0, st>>>(m, fpsiy, fcoly);
-            k_face_map_p<HV_GARM_P, 2, true><<<gz, 128, 0, st>>>(m, fpsiz, fcolz);
-        } else {
-            k_face_map_p<HV_GARM_P, 0, false><<<gx, 128, 0, st>>>(m, fpsix, fcolx);
-            k_face_map_p<HV_GARM_P, 1, false><<<gy, 128, 0, st>>>(m, fpsiy, fcoly);
-            k_face_map_p<HV_GARM_P, 2, false><<<gz, 128, 0, st>>>(m, fpsiz, fcolz);
-        }
+        if (m.pow2) k_face_map_rest<HV_GARM_P, true><<<r, 128, 0, st>>>(m, fp, fc, chunk);
+        else k_face_map_rest<HV_GARM_P, false><<<r, 128, 0, st>>>(m, fp, fc, chunk);
     } else {
-        if (m.pow2) {
-            k_face_map_p<HV_FULL, 0, true><<<gx, 128, 0, st>>>(m, fpsix, fcolx);
-            k_face_map_p<HV_FULL, 1, true><<<gy, 128, 0, st>>>(m, fpsiy, fcoly);
-            k_face_map_p<HV_FULL, 2, true><<<gz, 128, 0, st>>>(m, fpsiz, fcolz);
-        } else {
-            k_face_map_p<HV_FULL, 0, false><<<gx, 128, 0, st>>>(m, fpsix, fcolx);
-            k_face_map_p<HV_FULL, 1, false><<<gy, 128, 0, st>>>(m, fpsiy, fcoly);
-            k_face_map_p<HV_FULL, 2, false><<<gz, 128, 0, st>>>(m, fpsiz, fcolz);
-        }
+        if (m.pow2) k_face_map_rest<HV_FULL, true><<<r, 128, 0, st>>>(m, fp, fc, chunk);
+        else k_face_map_rest<HV_FULL, false><<<r, 128, 0, st>>>(m, fp, fc, chunk);
     }
     return launch_status();
 }
