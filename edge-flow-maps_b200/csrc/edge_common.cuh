@@ -66,14 +66,14 @@ EDGE_D f2 pair(float lo, float hi) {
 }
 EDGE_D f2 both(float a) { return pair(a, a); }
 EDGE_D float lo(f2 a) {
-    float x, y;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    float x;
+    asm("mov.b64 {%0, _}, %1;" : "=f"(x) : "l"(a.v));
     return x;
 }
 EDGE_D float hi(f2 a) {
-    float x, y;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
-    return y;
+    float x;
+    asm("mov.b64 {_, %0}, %1;" : "=f"(x) : "l"(a.v));
+    return x;
 }
 EDGE_D f2 fma2(f2 a, f2 b, f2 c) {
     f2 d;

@@ -430,6 +430,15 @@ int edge_lp_vel_diff(int nx, int ny, int nz, float dx, const float *ux, const fl
 int edge_lp_p2g(int nx, int ny, int nz, float dx, float *dragx, float *dragy, float *dragz, const float *vdiff,
                 const float *pos, const float *rad, int num, float laden_radius, float Lx, float Ly, float Lz,
                 void *stream);
+/* The same scatter with the particles grouped by cell first, their sums per
+ * cell formed before the atomic adds: the faster one where several particles
+ * share a cell.  work: device memory of at least the size that
+ * edge_lp_p2g_workspace gives, 16-byte aligned, free again when the call's
+ * work on the stream is done. */
+int edge_lp_p2g_workspace(int nx, int ny, int nz, int num, long long *bytes);
+int edge_lp_p2g_grouped(int nx, int ny, int nz, float dx, float *dragx, float *dragy, float *dragz,
+                        const float *vdiff, const float *pos, const float *rad, int num, float laden_radius,
+                        float Lx, float Ly, float Lz, void *work, long long work_bytes, void *stream);
 /* calc_max_particle_speed, run_edge.py:256-261: max |v| (>= 1e-3) of the
  * first num particles into out (one float, device memory) */
 int edge_lp_max_speed(const float *vel, int num, float *out, void *stream);
