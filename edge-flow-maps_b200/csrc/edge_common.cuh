@@ -85,6 +85,11 @@ EDGE_D f2 mul2(f2 a, f2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
     return d;
 }
+EDGE_D f2 add2(f2 a, f2 b) {
+    f2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+    return d;
+}
 // a0 b0 + a1 b1 + a2 b2 with the roundings of the scalar expression as nvcc
 // contracts it (the products of the inner sum: the first is fused)
 EDGE_D f2 dot3(f2 a0, f2 b0, f2 a1, f2 b1, f2 a2, f2 b2) { return fma2(a2, b2, fma2(a0, b0, mul2(a1, b1))); }
@@ -146,18 +151,32 @@ EDGE_D Axis3<GRAD> bspline_axis(float u, float hi_) {
     // third derivatives (2 |x| - 3) / 2 are x0 - 1.5 and x0 - 0.5.
     const float x1 = x0 - 1.0f, t0 = 1.5f - x0, t2 = x0 - 0.5f;
     set_tap(a.w[0], (0.5f * t0) * t0, x0 - 1.5f);
-    set_tap(a.w[1], 0.75f - x1 * x1, -2.0f * x1);
+    set_tap(a.w[1], __fmaf_rn(-x1, x1, 0.75f), -2.0f * x1);
     set_tap(a.w[2], (0.5f * t2) * t2, t2);
     return a;
 }
 
-// Row pointer of tap row (i, j): one 32-bit byte offset per sample added to
-// the row's uniform address, so that a row costs one add and its taps are
-// immediate offsets.  BIG: grids whose faces may pass 4 GB per component.
+// Tap row (i, j) of a sample, tap k by [k].  In global memory: one 32-bit byte
+// offset per sample added to the row's uniform address, so that a row costs
+// one add and its taps are immediate offsets.  BIG: grids whose faces may pass
+// 4 GB per component.
+struct GRow {
+    const float* p;
+    EDGE_D float operator[](int k) const { return __ldg(p + k); }
+};
 template <bool BIG>
-EDGE_D const float* tap_row(const float* f, int e, int i, int j, int n1, int n2) {
-    if (BIG) return f + e + (i * n1 + j) * n2;
-    return reinterpret_cast<const float*>(reinterpret_cast<const char*>(f + (i * n1 + j) * n2) + 4u * (unsigned)e);
+struct GRows {
+    const float* f;
+    int e, n1, n2;
+    EDGE_D GRow operator()(int i, int j) const {
+        if (BIG) return GRow{f + e + (i * n1 + j) * n2};
+        return GRow{reinterpret_cast<const float*>(reinterpret_cast<const char*>(f + (i * n1 + j) * n2) +
+                                                   4u * (unsigned)e)};
+    }
+};
+template <bool BIG>
+EDGE_D GRows<BIG> grows(const float* f, int x, int y, int z, int n1, int n2) {
+    return GRows<BIG>{f, idx3(x, y, z, n1, n2), n1, n2};
 }
 
 // 27-tap separable contraction of one scalar field, z then y then x, value and
@@ -168,20 +187,19 @@ EDGE_D const float* tap_row(const float* f, int e, int i, int j, int n1, int n2)
 // instructions per three-component sample with scalar multiply-adds and 64-bit
 // row addresses, 515 in this form (RK4 with Jacobian of 128^3 cells, 12
 // samples each: 0.611 -> 0.508 ms, the same bits).
-template <bool BIG>
-EDGE_D float bspline_sum(const float* __restrict__ f, int n1, int n2, const Axis3<true>& X, const Axis3<true>& Y,
-                         const Axis3<true>& Z, float inv_dx, float* g) {
+template <class Rows>
+EDGE_D float bspline_sum(const Rows& rows, const Axis3<true>& X, const Axis3<true>& Y, const Axis3<true>& Z,
+                         float inv_dx, float* g) {
     f2 vz = both(0.0f);  // (value, z derivative)
     float gx = 0.0f, gy = 0.0f;
-    const int e = idx3(X.base, Y.base, Z.base, n1, n2);
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         f2 c = both(0.0f);
         float cy = 0.0f;
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            const float* row = tap_row<BIG>(f, e, i, j, n1, n2);
-            const f2 a = dot3(Z.w[0], both(__ldg(row)), Z.w[1], both(__ldg(row + 1)), Z.w[2], both(__ldg(row + 2)));
+            const auto q = rows(i, j);
+            const f2 a = dot3(Z.w[0], both(q[0]), Z.w[1], both(q[1]), Z.w[2], both(q[2]));
             c = fma2(both(lo(Y.w[j])), a, c);
             cy = __fmaf_rn(hi(Y.w[j]), lo(a), cy);
         }
@@ -200,26 +218,25 @@ EDGE_D float bspline_sum(const float* __restrict__ f, int n1, int n2, const Axis
 // 27 taps are loaded before the first is used: the kernels that take one
 // sample per thread wait for their gathers (velocity pullback at 256x128x128
 // 344 us row by row, 322 us so, 343 us with the scalar sampler).
-template <bool BIG>
-EDGE_D float bspline_sum(const float* __restrict__ f, int n1, int n2, const Axis3<false>& X, const Axis3<false>& Y,
-                         const Axis3<false>& Z, float, float*) {
-    const int e = idx3(X.base, Y.base, Z.base, n1, n2);
+template <class Rows>
+EDGE_D float bspline_sum(const Rows& rows, const Axis3<false>& X, const Axis3<false>& Y, const Axis3<false>& Z, float,
+                         float*) {
     float q[3][3][3];
 #pragma unroll
     for (int i = 0; i < 3; i++)
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-            const float* row = tap_row<BIG>(f, e, i, j, n1, n2);
+            const auto row = rows(i, j);
 #pragma unroll
-            for (int k = 0; k < 3; k++) q[i][j][k] = __ldg(row + k);
+            for (int k = 0; k < 3; k++) q[i][j][k] = row[k];
         }
-    auto rows = [&](const float (&a)[3], const float (&b)[3]) {
+    auto pairs = [&](const float (&a)[3], const float (&b)[3]) {
         return dot3(both(Z.w[0]), pair(a[0], b[0]), both(Z.w[1]), pair(a[1], b[1]), both(Z.w[2]), pair(a[2], b[2]));
     };
     f2 c01 = both(0.0f);
 #pragma unroll
-    for (int j = 0; j < 3; j++) c01 = fma2(both(Y.w[j]), rows(q[0][j], q[1][j]), c01);
-    const f2 a2 = rows(q[2][0], q[2][1]);
+    for (int j = 0; j < 3; j++) c01 = fma2(both(Y.w[j]), pairs(q[0][j], q[1][j]), c01);
+    const f2 a2 = pairs(q[2][0], q[2][1]);
     float c2 = __fmaf_rn(Y.w[0], lo(a2), 0.0f);
     c2 = __fmaf_rn(Y.w[1], hi(a2), c2);
     c2 = __fmaf_rn(Y.w[2], dot3(Z.w[0], q[2][2][0], Z.w[1], q[2][2][1], Z.w[2], q[2][2][2]), c2);
@@ -251,36 +268,174 @@ static inline Mac make_mac(const float* ux, const float* uy, const float* uz, in
     return m;
 }
 
+// The six axes of a sample at p: A0 where the component is normal to the axis,
+// A5 where it is tangential.
+template <bool GRAD>
+EDGE_D void mac_axes(const Mac& m, const float p[3], float q[3], Axis3<GRAD> A0[3], Axis3<GRAD> A5[3]) {
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        q[d] = over_dx(p[d], m.dx, m.inv_dx, m.pow2);
+        A0[d] = bspline_axis<GRAD>(q[d], m.hi0[d]);
+        A5[d] = bspline_axis<GRAD>(q[d] - 0.5f, m.hi5[d]);
+    }
+}
+template <bool GRAD, bool BIG>
+EDGE_D void mac_sums(const Mac& m, const Axis3<GRAD> A0[3], const Axis3<GRAD> A5[3], float v[3], float G[3][3]) {
+    v[0] = bspline_sum(grows<BIG>(m.u[0], A0[0].base, A5[1].base, A5[2].base, m.ny, m.nz), A0[0], A5[1], A5[2],
+                       m.inv_dx, GRAD ? G[0] : nullptr);
+    v[1] = bspline_sum(grows<BIG>(m.u[1], A5[0].base, A0[1].base, A5[2].base, m.ny + 1, m.nz), A5[0], A0[1], A5[2],
+                       m.inv_dx, GRAD ? G[1] : nullptr);
+    v[2] = bspline_sum(grows<BIG>(m.u[2], A5[0].base, A5[1].base, A0[2].base, m.ny, m.nz + 1), A5[0], A5[1], A0[2],
+                       m.inv_dx, GRAD ? G[2] : nullptr);
+}
+
 // interp_u_MAC / interp_u_MAC_grad (taichi_utils.py:322-341).  G rows are the
 // gradients of u_x, u_y, u_z.
 template <bool GRAD, bool BIG = false>
 EDGE_D void mac_sample(const Mac& m, const float p[3], float v[3], float G[3][3]) {
-    float q[3] = {over_dx(p[0], m.dx, m.inv_dx, m.pow2), over_dx(p[1], m.dx, m.inv_dx, m.pow2),
-                  over_dx(p[2], m.dx, m.inv_dx, m.pow2)};
+    float q[3];
     Axis3<GRAD> A0[3], A5[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        A0[d] = bspline_axis<GRAD>(q[d], m.hi0[d]);
-        A5[d] = bspline_axis<GRAD>(q[d] - 0.5f, m.hi5[d]);
-    }
-    v[0] = bspline_sum<BIG>(m.u[0], m.ny, m.nz, A0[0], A5[1], A5[2], m.inv_dx, GRAD ? G[0] : nullptr);
-    v[1] = bspline_sum<BIG>(m.u[1], m.ny + 1, m.nz, A5[0], A0[1], A5[2], m.inv_dx, GRAD ? G[1] : nullptr);
-    v[2] = bspline_sum<BIG>(m.u[2], m.ny, m.nz + 1, A5[0], A5[1], A0[2], m.inv_dx, GRAD ? G[2] : nullptr);
+    mac_axes<GRAD>(m, p, q, A0, A5);
+    mac_sums<GRAD, BIG>(m, A0, A5, v, G);
 }
 
 // Component a of interp_u_MAC alone (mac_sample's arithmetic for that
 // component): the semi-Lagrangian advection keeps only the face's own
 // component of its last sample.
 EDGE_D float mac_sample_comp(const Mac& m, const float p[3], int a) {
-    float q[3] = {over_dx(p[0], m.dx, m.inv_dx, m.pow2), over_dx(p[1], m.dx, m.inv_dx, m.pow2),
-                  over_dx(p[2], m.dx, m.inv_dx, m.pow2)};
     Axis3<false> A[3];
 #pragma unroll
-    for (int d = 0; d < 3; d++)
-        A[d] = d == a ? bspline_axis<false>(q[d], m.hi0[d]) : bspline_axis<false>(q[d] - 0.5f, m.hi5[d]);
-    if (a == 0) return bspline_sum<false>(m.u[0], m.ny, m.nz, A[0], A[1], A[2], m.inv_dx, nullptr);
-    if (a == 1) return bspline_sum<false>(m.u[1], m.ny + 1, m.nz, A[0], A[1], A[2], m.inv_dx, nullptr);
-    return bspline_sum<false>(m.u[2], m.ny, m.nz + 1, A[0], A[1], A[2], m.inv_dx, nullptr);
+    for (int d = 0; d < 3; d++) {
+        const float q = over_dx(p[d], m.dx, m.inv_dx, m.pow2);
+        A[d] = d == a ? bspline_axis<false>(q, m.hi0[d]) : bspline_axis<false>(q - 0.5f, m.hi5[d]);
+    }
+    const int n1 = m.ny + (a == 1), n2 = m.nz + (a == 2);
+    const float* u = a == 0 ? m.u[0] : (a == 1 ? m.u[1] : m.u[2]);
+    return bspline_sum(grows<false>(u, A[0].base, A[1].base, A[2].base, n1, n2), A[0], A[1], A[2], m.inv_dx, nullptr);
+}
+
+// ---------------------------------------------------------------------------
+// The velocity around a block of TI x TJ x TK cells in shared memory, for the
+// marches that take some ten samples within a cell of where they start.  Row
+// strides are constants there, so a tap is one instruction, and a warp's 32
+// consecutive taps are one wavefront at any alignment (1.43 in global memory).
+// Two nodes on each side of the block hold every tap of a sample whose
+// coordinate is in (i - 1, i + 1.5) on each axis, i the thread's cell: tap
+// nodes floor(q - 0.5) .. + 2 and, staggered, floor(q - 1) .. + 2, and the
+// clamped ones near the walls (a cell index is at most n - 1).  A warp with a
+// sample outside that takes it from global memory.
+// ---------------------------------------------------------------------------
+// Blocks of 4 x 4 x 8 cells: 2 x 2 x 32 stage more nodes per cell, were slower
+// and leave more of a ragged grid's threads idle.
+template <int TI, int TJ, int TK>
+struct Tile {
+    static constexpr int I = TI, J = TJ, K = TK, threads = TI * TJ * TK;
+    static constexpr int N0 = TI + 4, N1 = TJ + 4, N2 = TK + 4;
+    // rows of eight cells: the four rows of a warp start 24 words apart, 0, 24,
+    // 16, 8 modulo 32, and a row holds two components' twelve nodes
+    static_assert(TK == 8, "two components per row of 24 words");
+    static constexpr int S2 = 2 * N2, S1 = N1 * S2;
+    static constexpr int at(int a) { return a == 1 ? N2 : (a == 2 ? N0 * S1 : 0); }
+    static constexpr int size = 2 * N0 * S1;
+};
+struct SRow {
+    const float* p;
+    EDGE_D float operator[](int k) const { return p[k]; }
+};
+template <class T>
+struct SRows {
+    const float* p;
+    EDGE_D SRow operator()(int i, int j) const { return SRow{p + i * T::S1 + j * T::S2}; }
+};
+template <class T>
+struct MacTile {
+    Mac m;
+    const float* sm;  // component a at T::at(a)
+    int off;          // node (0, 0, 0) is at sm - off
+    float c[3];       // the thread's cell + 0.25
+    unsigned mask;    // the warp's threads that sample
+    EDGE_D SRows<T> rows(int a, int x, int y, int z) const {
+        return SRows<T>{sm + T::at(a) + ((x * T::N1 + y) * T::S2 + z - off)};
+    }
+    EDGE_D bool holds(const float q[3]) const {
+        const bool in = fabsf(q[0] - c[0]) < 1.25f && fabsf(q[1] - c[1]) < 1.25f && fabsf(q[2] - c[2]) < 1.25f;
+        return __all_sync(mask, in);
+    }
+};
+// thread 16 b + c loads node (a, b, c) of every plane a
+template <class T>
+EDGE_D void stage_tile(const Mac& m, float* sm, int i0, int j0, int k0) {
+    static_assert(T::N1 * 16 == T::threads && T::N2 <= 16, "sixteen threads per row of nodes");
+    const int c = threadIdx.x & 15, b = threadIdx.x >> 4;
+    if (c >= T::N2) return;
+    const int j = max(j0 - 2 + b, 0), k = max(k0 - 2 + c, 0);
+    const int jc = min(j, m.ny - 1), kc = min(k, m.nz - 1);
+    const float* ux = m.u[0] + jc * m.nz + kc;
+    const float* uy = m.u[1] + min(j, m.ny) * m.nz + kc;
+    const float* uz = m.u[2] + jc * (m.nz + 1) + min(k, m.nz);
+    float* d = sm + b * T::S2 + c;
+#pragma unroll
+    for (int a = 0; a < T::N0; a++) {
+        const int i = max(i0 - 2 + a, 0), ic = min(i, m.nx - 1);
+        d[T::at(0) + a * T::S1] = __ldg(ux + min(i, m.nx) * (m.ny * m.nz));
+        d[T::at(1) + a * T::S1] = __ldg(uy + ic * ((m.ny + 1) * m.nz));
+        d[T::at(2) + a * T::S1] = __ldg(uz + ic * (m.ny * (m.nz + 1)));
+    }
+}
+// Stages cell tile `block` (in k, j, i order over the grid) and finds the
+// thread's cell; false for a thread past the grid.  All threads of the block.
+template <class T>
+EDGE_D bool enter_tile(const Mac& m, float* sm, unsigned block, MacTile<T>& t, int& i, int& j, int& k) {
+    const unsigned nk = (unsigned)(m.nz + T::K - 1) / T::K, nj = (unsigned)(m.ny + T::J - 1) / T::J;
+    const unsigned bj = block / nk, bi = bj / nj;
+    const int k0 = (int)(block - bj * nk) * T::K, j0 = (int)(bj - bi * nj) * T::J, i0 = (int)bi * T::I;
+    stage_tile<T>(m, sm, i0, j0, k0);
+    __syncthreads();
+    k = k0 + (int)threadIdx.x % T::K;
+    j = j0 + (int)threadIdx.x / T::K % T::J;
+    i = i0 + (int)threadIdx.x / (T::K * T::J);
+    const bool in = i < m.nx && j < m.ny && k < m.nz;
+    t.m = m;
+    t.sm = sm;
+    t.off = ((i0 - 2) * T::N1 + (j0 - 2)) * T::S2 + (k0 - 2);
+    t.c[0] = (float)i + 0.25f;
+    t.c[1] = (float)j + 0.25f;
+    t.c[2] = (float)k + 0.25f;
+    t.mask = __ballot_sync(0xffffffffu, in);
+    return in;
+}
+template <class T>
+static inline int tile_blocks(int nx, int ny, int nz) {
+    return (nx + T::I - 1) / T::I * ((ny + T::J - 1) / T::J) * ((nz + T::K - 1) / T::K);
+}
+template <class T>
+EDGE_D float mac_sample_comp(const MacTile<T>& t, const float p[3], int a) {
+    float q[3];
+    Axis3<false> A[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        q[d] = over_dx(p[d], t.m.dx, t.m.inv_dx, t.m.pow2);
+        A[d] = d == a ? bspline_axis<false>(q[d], t.m.hi0[d]) : bspline_axis<false>(q[d] - 0.5f, t.m.hi5[d]);
+    }
+    if (t.holds(q))
+        return bspline_sum(t.rows(a, A[0].base, A[1].base, A[2].base), A[0], A[1], A[2], t.m.inv_dx, nullptr);
+    return mac_sample_comp(t.m, p, a);
+}
+template <bool GRAD, class T>
+EDGE_D void mac_sample(const MacTile<T>& t, const float p[3], float v[3], float G[3][3]) {
+    float q[3];
+    Axis3<GRAD> A0[3], A5[3];
+    mac_axes<GRAD>(t.m, p, q, A0, A5);
+    if (t.holds(q)) {
+        v[0] = bspline_sum(t.rows(0, A0[0].base, A5[1].base, A5[2].base), A0[0], A5[1], A5[2], t.m.inv_dx,
+                           GRAD ? G[0] : nullptr);
+        v[1] = bspline_sum(t.rows(1, A5[0].base, A0[1].base, A5[2].base), A5[0], A0[1], A5[2], t.m.inv_dx,
+                           GRAD ? G[1] : nullptr);
+        v[2] = bspline_sum(t.rows(2, A5[0].base, A5[1].base, A0[2].base), A5[0], A5[1], A0[2], t.m.inv_dx,
+                           GRAD ? G[2] : nullptr);
+    } else {
+        mac_sums<GRAD, false>(t.m, A0, A5, v, G);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -699,33 +854,179 @@ EDGE_D void hermite3p(const MapP& m, const float p[3], float val[3], float grad[
     }
 }
 
+// The 8 Hermite coefficients of one corner, bit 2 / 1 / 0 of the index = the g
+// basis along x / y / z, components x and y as a pair.
+struct HCorner {
+    f2 xy[8];
+    float z[8];
+};
+EDGE_D void set_coef(HCorner& t, int q, const float4& v) {
+    t.xy[q] = pair(v.x, v.y);
+    t.z[q] = v.z;
+}
+EDGE_D void set_coef(HCorner& t, int q, const float4& v, float s) {
+    t.xy[q] = mul2(pair(v.x, v.y), both(s));
+    t.z[q] = v.z * s;
+}
+// hcoef_p and hcoef_p_unscaled
+template <int VARIANT>
+EDGE_D void hcorner(const MapP& m, int e, HCorner& t) {
+    const float dx = m.dx;
+    set_coef(t, 0, ldp(m, 0, e));
+    set_coef(t, 4, ldp(m, 1, e), dx);
+    set_coef(t, 2, ldp(m, 2, e), dx);
+    set_coef(t, 1, ldp(m, 3, e), dx);
+    constexpr int slot[4] = {3, 5, 6, 7};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        set_coef(t, slot[q], ldp(m, 4 + q, e), dx);
+        if (VARIANT != HV_FD_P) {
+            const int more = q == 3 && VARIANT == HV_FULL ? 2 : 1;
+#pragma unroll
+            for (int r = 0; r < more; r++) {
+                t.xy[slot[q]] = mul2(t.xy[slot[q]], both(dx));
+                t.z[slot[q]] = t.z[slot[q]] * dx;
+            }
+        }
+    }
+}
+
+template <int VARIANT>
+EDGE_D void hcorner_unscaled(const MapP& m, int e, HCorner& t) {
+    const float inv = m.inv_dx;
+    set_coef(t, 0, ldp(m, 0, e));
+    set_coef(t, 4, ldp(m, 1, e));
+    set_coef(t, 2, ldp(m, 2, e));
+    set_coef(t, 1, ldp(m, 3, e));
+    if (VARIANT == HV_FD_P) {  // planes 4-7 hold the terms over dx (hcoef_p multiplies by dx once)
+        set_coef(t, 3, ldp(m, 4, e), inv);
+        set_coef(t, 5, ldp(m, 5, e), inv);
+        set_coef(t, 6, ldp(m, 6, e), inv);
+        set_coef(t, 7, ldp(m, 7, e), inv);
+        t.xy[7] = mul2(t.xy[7], both(inv));
+        t.z[7] = t.z[7] * inv;
+    } else {
+        set_coef(t, 3, ldp(m, 4, e));
+        set_coef(t, 5, ldp(m, 5, e));
+        set_coef(t, 6, ldp(m, 6, e));
+        if (VARIANT == HV_GARM_P) set_coef(t, 7, ldp(m, 7, e), inv);  // plane 7 holds psi_xyz over dx
+        else set_coef(t, 7, ldp(m, 7, e));
+    }
+}
+
+// f a + g b (+ acc) with the roundings of the scalar expressions as nvcc
+// contracts them
+EDGE_D float mix(float f, float a, float g, float b) { return __fmaf_rn(f, a, __fmul_rn(g, b)); }
+EDGE_D f2 mix(float f, f2 a, float g, f2 b) { return fma2(both(f), a, mul2(both(g), b)); }
+EDGE_D float mix(float f, float a, float g, float b, float acc) { return __fadd_rn(acc, mix(f, a, g, b)); }
+EDGE_D f2 mix(float f, f2 a, float g, f2 b, f2 acc) { return add2(acc, mix(f, a, g, b)); }
+
+// The contraction of one corner for one component (T = float) or two (f2).
+template <class T>
+EDGE_D void hcontract(const T t[8], const HAxis& Y, const HAxis& Z, int j, int k, T (&A)[2], T (&B)[2], T (&dA)[2]) {
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+        const T P0 = mix(Z.f[k], t[a * 4 + 0], Z.g[k], t[a * 4 + 1]);
+        const T P1 = mix(Z.f[k], t[a * 4 + 2], Z.g[k], t[a * 4 + 3]);
+        A[a] = mix(Y.f[j], P0, Y.g[j], P1, A[a]);
+        B[a] = mix(Y.df[j], P0, Y.dg[j], P1, B[a]);
+        const T dP0 = mix(Z.df[k], t[a * 4 + 0], Z.dg[k], t[a * 4 + 1]);
+        const T dP1 = mix(Z.df[k], t[a * 4 + 2], Z.dg[k], t[a * 4 + 3]);
+        dA[a] = mix(Y.f[j], dP0, Y.g[j], dP1, dA[a]);
+    }
+}
+
+// hermite3p with the gradient, components x and y as pairs: the same values
+// with two thirds of the contraction's issue slots, for more registers; what
+// it gives depends on the register cap.  EDGE march at 4 blocks of 128 threads
+// per SM: 256x128x128 2979 us in the scalar form at its best, 2684 us so; GE
+// march at 5 blocks: 96^3 184 -> 166 us.  The value alone is better off in the
+// scalar form (ED8 march 2967 against 3169 us).
+template <int VARIANT>
+EDGE_D void hermite3p_pairs(const MapP& m, const float p[3], float val[3], float grad[3][3]) {
+    float q[3] = {over_dx(p[0], m.dx, m.inv_dx, m.pow2) - 0.5f, over_dx(p[1], m.dx, m.inv_dx, m.pow2) - 0.5f,
+                  over_dx(p[2], m.dx, m.inv_dx, m.pow2) - 0.5f};
+    HAxis X = haxis(q[0], m.hi[0], m.nx), Y = haxis(q[1], m.hi[1], m.ny), Z = haxis(q[2], m.hi[2], m.nz);
+    // power-of-two dx: the g basis functions carry dx and the coefficients
+    // come unscaled (hcoef_p_unscaled); the same products, fewer multiplies
+    const bool fold = m.pow2;
+    if (fold) {
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            X.g[c] *= m.dx; X.dg[c] *= m.dx;
+            Y.g[c] *= m.dx; Y.dg[c] *= m.dx;
+            Z.g[c] *= m.dx; Z.dg[c] *= m.dx;
+        }
+    }
+    f2 v2 = both(0.f), gx2 = v2, gy2 = v2, gz2 = v2;       // components x, y
+    float v1 = 0.f, gx1 = 0.f, gy1 = 0.f, gz1 = 0.f;       // component z
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int ii = i ? X.cp : X.c0;
+        f2 A2[2] = {both(0.f), both(0.f)}, B2[2] = {both(0.f), both(0.f)}, dA2[2] = {both(0.f), both(0.f)};
+        float A1[2] = {0.f, 0.f}, B1[2] = {0.f, 0.f}, dA1[2] = {0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int jj = j ? Y.cp : Y.c0;
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int kk = k ? Z.cp : Z.c0;
+                HCorner t;
+                if (fold) hcorner_unscaled<VARIANT>(m, idx3(ii, jj, kk, m.ny, m.nz), t);
+                else hcorner<VARIANT>(m, idx3(ii, jj, kk, m.ny, m.nz), t);
+                hcontract(t.xy, Y, Z, j, k, A2, B2, dA2);
+                hcontract(t.z, Y, Z, j, k, A1, B1, dA1);
+            }
+        }
+        v2 = mix(X.f[i], A2[0], X.g[i], A2[1], v2);
+        v1 = mix(X.f[i], A1[0], X.g[i], A1[1], v1);
+        gx2 = mix(X.df[i], A2[0], X.dg[i], A2[1], gx2);
+        gx1 = mix(X.df[i], A1[0], X.dg[i], A1[1], gx1);
+        gy2 = mix(X.f[i], B2[0], X.g[i], B2[1], gy2);
+        gy1 = mix(X.f[i], B1[0], X.g[i], B1[1], gy1);
+        gz2 = mix(X.f[i], dA2[0], X.g[i], dA2[1], gz2);
+        gz1 = mix(X.f[i], dA1[0], X.g[i], dA1[1], gz1);
+    }
+    val[0] = lo(v2); val[1] = hi(v2); val[2] = v1;
+    const float inv = 1.0f / m.dx;
+    grad[0][0] = lo(gx2) * inv; grad[1][0] = hi(gx2) * inv; grad[2][0] = gx1 * inv;
+    grad[0][1] = lo(gy2) * inv; grad[1][1] = hi(gy2) * inv; grad[2][1] = gy1 * inv;
+    grad[0][2] = lo(gz2) * inv; grad[1][2] = hi(gz2) * inv; grad[2][2] = gz1 * inv;
+}
+
 // ---------------------------------------------------------------------------
 // RK4 marches (hermite.py:786-860, run_edge.py:337-357)
 // ---------------------------------------------------------------------------
-EDGE_D void rk4_pos(const Mac& mac, float psi[3], float dt) {
-    float u1[3], u2[3], u3[3], u4[3], q[3];
-    float h = 0.5f * dt;
-    mac_sample<false>(mac, psi, u1, nullptr);
+// M: Mac or MacTile.  The stages run as a loop: one copy of the sampler keeps
+// the kernels inside the instruction cache.
+template <class M>
+EDGE_D void rk4_pos(const M& mac, float psi[3], float dt) {
+    float u[3], q[3], su[3] = {0.0f, 0.0f, 0.0f};
+    const float h = 0.5f * dt;
 #pragma unroll
-    for (int c = 0; c < 3; c++) q[c] = psi[c] + h * u1[c];
-    mac_sample<false>(mac, q, u2, nullptr);
+    for (int c = 0; c < 3; c++) q[c] = psi[c];
+#pragma unroll 1
+    for (int stage = 0; stage < 4; stage++) {
+        mac_sample<false>(mac, q, u, nullptr);
+        const float wt = (stage == 0 || stage == 3) ? 1.0f : 2.0f;
+        const float hh = stage < 2 ? h : dt;
 #pragma unroll
-    for (int c = 0; c < 3; c++) q[c] = psi[c] + h * u2[c];
-    mac_sample<false>(mac, q, u3, nullptr);
+        for (int c = 0; c < 3; c++) {
+            su[c] = __fmaf_rn(wt, u[c], su[c]);
+            q[c] = __fmaf_rn(hh, u[c], psi[c]);
+        }
+    }
+    const float w6 = dt * 1.0f / 6.0f;
 #pragma unroll
-    for (int c = 0; c < 3; c++) q[c] = psi[c] + dt * u3[c];
-    mac_sample<false>(mac, q, u4, nullptr);
-    float w6 = dt * 1.0f / 6.0f;
-#pragma unroll
-    for (int c = 0; c < 3; c++) psi[c] = psi[c] + w6 * (u1[c] + 2.0f * u2[c] + 2.0f * u3[c] + u4[c]);
+    for (int c = 0; c < 3; c++) psi[c] = __fmaf_rn(w6, su[c], psi[c]);
 }
 
 // RK4 of a point with NC Jacobian columns C[a] (dC/dt = grad u . C).  The
 // four stages run as a loop (not unrolled): one copy of the 81-tap sampler
 // keeps the kernels inside the instruction cache.  Columns 0 and 1 are
 // advanced as pairs.
-template <int NC>
-EDGE_D void rk4_jac(const Mac& mac, float psi[3], float C[NC][3], float dt) {
+template <int NC, class M>
+EDGE_D void rk4_jac(const M& mac, float psi[3], float C[NC][3], float dt) {
     static_assert(NC == 1 || NC == 3, "one column, or all three");
     constexpr int L = NC - 1;  // the column advanced on its own
     float u[3], G[3][3], q[3], su[3], s1[3], S1[3];
@@ -781,15 +1082,17 @@ EDGE_D void rk4_jac(const Mac& mac, float psi[3], float C[NC][3], float dt) {
     }
 }
 
+// products rounded on their own: contracted into a sum that follows (an epsilon
+// point), they would round otherwise where dx is no power of two
 EDGE_D void cell_pos(int i, int j, int k, float dx, float X[3]) {
-    X[0] = ((float)i + 0.5f) * dx;
-    X[1] = ((float)j + 0.5f) * dx;
-    X[2] = ((float)k + 0.5f) * dx;
+    X[0] = __fmul_rn((float)i + 0.5f, dx);
+    X[1] = __fmul_rn((float)j + 0.5f, dx);
+    X[2] = __fmul_rn((float)k + 0.5f, dx);
 }
 EDGE_D void face_pos(int axis, int i, int j, int k, float dx, float X[3]) {
-    X[0] = ((float)i + (axis == 0 ? 0.0f : 0.5f)) * dx;
-    X[1] = ((float)j + (axis == 1 ? 0.0f : 0.5f)) * dx;
-    X[2] = ((float)k + (axis == 2 ? 0.0f : 0.5f)) * dx;
+    X[0] = __fmul_rn((float)i + (axis == 0 ? 0.0f : 0.5f), dx);
+    X[1] = __fmul_rn((float)j + (axis == 1 ? 0.0f : 0.5f), dx);
+    X[2] = __fmul_rn((float)k + (axis == 2 ? 0.0f : 0.5f), dx);
 }
 
 // Decompose a linear face index over the three face grids (x faces first).
