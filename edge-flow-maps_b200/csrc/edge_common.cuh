@@ -157,26 +157,54 @@ EDGE_D Axis3<GRAD> bspline_axis(float u, float hi_) {
 }
 
 // Tap row (i, j) of a sample, tap k by [k].  In global memory: one 32-bit byte
-// offset per sample added to the row's uniform address, so that a row costs
-// one add and its taps are immediate offsets.  BIG: grids whose faces may pass
-// 4 GB per component.
+// offset per sample (grids have less than 2^30 faces per component) added to
+// the row's uniform address, so that a row costs one add and its taps are
+// immediate offsets.
 struct GRow {
     const float* p;
     EDGE_D float operator[](int k) const { return __ldg(p + k); }
 };
-template <bool BIG>
 struct GRows {
     const float* f;
     int e, n1, n2;
     EDGE_D GRow operator()(int i, int j) const {
-        if (BIG) return GRow{f + e + (i * n1 + j) * n2};
         return GRow{reinterpret_cast<const float*>(reinterpret_cast<const char*>(f + (i * n1 + j) * n2) +
                                                    4u * (unsigned)e)};
     }
 };
-template <bool BIG>
-EDGE_D GRows<BIG> grows(const float* f, int x, int y, int z, int n1, int n2) {
-    return GRows<BIG>{f, idx3(x, y, z, n1, n2), n1, n2};
+EDGE_D GRows grows(const float* f, int x, int y, int z, int n1, int n2) {
+    return GRows{f, idx3(x, y, z, n1, n2), n1, n2};
+}
+
+// The taps of samples at scattered points.  A warp's load there costs a
+// wavefront for every point or two, whatever its width, and 81 of them per
+// point were the bound: a row's three taps come in the aligned 16 bytes that
+// hold the first and, where these do not hold the third, the 8 bytes after
+// them.  `wide`: no such load passes either end of the field.  200 000 points
+// at random in 256x128x128 39 -> 32.5 us.
+struct VRow {
+    float q[3];
+    EDGE_D float operator[](int k) const { return q[k]; }
+};
+struct VRows {
+    const float* f;  // the sample's first tap
+    int n1, n2;
+    bool wide;
+    EDGE_D VRow operator()(int i, int j) const {
+        const float* p = f + (i * n1 + j) * n2;
+        if (!wide) return VRow{{__ldg(p), __ldg(p + 1), __ldg(p + 2)}};
+        const unsigned o = (unsigned)(reinterpret_cast<size_t>(p) >> 2) & 3;
+        const float4 a = __ldg(reinterpret_cast<const float4*>(p - o));
+        float2 b = make_float2(0.f, 0.f);
+        if (o >= 2) b = __ldg(reinterpret_cast<const float2*>(p - o + 4));
+        const float s0 = (o & 1) ? a.y : a.x, s1 = (o & 1) ? a.z : a.y, s2 = (o & 1) ? a.w : a.z, s3 = (o & 1) ? b.x : a.w;
+        const float s4 = (o & 1) ? b.y : b.x;
+        return (o & 2) ? VRow{{s2, s3, s4}} : VRow{{s0, s1, s2}};
+    }
+};
+EDGE_D VRows vrows(const float* f, int x, int y, int z, int n0, int n1, int n2) {
+    const long long e = ((long long)x * n1 + y) * n2 + z, last = e + (2LL * n1 + 2) * n2 + 2;
+    return VRows{f + e, n1, n2, e >= 3 && last + 3 < (long long)n0 * n1 * n2};
 }
 
 // 27-tap separable contraction of one scalar field, z then y then x, value and
@@ -279,24 +307,37 @@ EDGE_D void mac_axes(const Mac& m, const float p[3], float q[3], Axis3<GRAD> A0[
         A5[d] = bspline_axis<GRAD>(q[d] - 0.5f, m.hi5[d]);
     }
 }
-template <bool GRAD, bool BIG>
+template <bool GRAD>
 EDGE_D void mac_sums(const Mac& m, const Axis3<GRAD> A0[3], const Axis3<GRAD> A5[3], float v[3], float G[3][3]) {
-    v[0] = bspline_sum(grows<BIG>(m.u[0], A0[0].base, A5[1].base, A5[2].base, m.ny, m.nz), A0[0], A5[1], A5[2],
+    v[0] = bspline_sum(grows(m.u[0], A0[0].base, A5[1].base, A5[2].base, m.ny, m.nz), A0[0], A5[1], A5[2],
                        m.inv_dx, GRAD ? G[0] : nullptr);
-    v[1] = bspline_sum(grows<BIG>(m.u[1], A5[0].base, A0[1].base, A5[2].base, m.ny + 1, m.nz), A5[0], A0[1], A5[2],
+    v[1] = bspline_sum(grows(m.u[1], A5[0].base, A0[1].base, A5[2].base, m.ny + 1, m.nz), A5[0], A0[1], A5[2],
                        m.inv_dx, GRAD ? G[1] : nullptr);
-    v[2] = bspline_sum(grows<BIG>(m.u[2], A5[0].base, A5[1].base, A0[2].base, m.ny, m.nz + 1), A5[0], A5[1], A0[2],
+    v[2] = bspline_sum(grows(m.u[2], A5[0].base, A5[1].base, A0[2].base, m.ny, m.nz + 1), A5[0], A5[1], A0[2],
                        m.inv_dx, GRAD ? G[2] : nullptr);
+}
+
+// interp_u_MAC at a scattered point.
+EDGE_D void mac_sample_points(const Mac& m, const float p[3], float v[3]) {
+    float q[3];
+    Axis3<false> A0[3], A5[3];
+    mac_axes<false>(m, p, q, A0, A5);
+    v[0] = bspline_sum(vrows(m.u[0], A0[0].base, A5[1].base, A5[2].base, m.nx + 1, m.ny, m.nz), A0[0], A5[1], A5[2],
+                       m.inv_dx, nullptr);
+    v[1] = bspline_sum(vrows(m.u[1], A5[0].base, A0[1].base, A5[2].base, m.nx, m.ny + 1, m.nz), A5[0], A0[1], A5[2],
+                       m.inv_dx, nullptr);
+    v[2] = bspline_sum(vrows(m.u[2], A5[0].base, A5[1].base, A0[2].base, m.nx, m.ny, m.nz + 1), A5[0], A5[1], A0[2],
+                       m.inv_dx, nullptr);
 }
 
 // interp_u_MAC / interp_u_MAC_grad (taichi_utils.py:322-341).  G rows are the
 // gradients of u_x, u_y, u_z.
-template <bool GRAD, bool BIG = false>
+template <bool GRAD>
 EDGE_D void mac_sample(const Mac& m, const float p[3], float v[3], float G[3][3]) {
     float q[3];
     Axis3<GRAD> A0[3], A5[3];
     mac_axes<GRAD>(m, p, q, A0, A5);
-    mac_sums<GRAD, BIG>(m, A0, A5, v, G);
+    mac_sums<GRAD>(m, A0, A5, v, G);
 }
 
 // Component a of interp_u_MAC alone (mac_sample's arithmetic for that
@@ -311,7 +352,7 @@ EDGE_D float mac_sample_comp(const Mac& m, const float p[3], int a) {
     }
     const int n1 = m.ny + (a == 1), n2 = m.nz + (a == 2);
     const float* u = a == 0 ? m.u[0] : (a == 1 ? m.u[1] : m.u[2]);
-    return bspline_sum(grows<false>(u, A[0].base, A[1].base, A[2].base, n1, n2), A[0], A[1], A[2], m.inv_dx, nullptr);
+    return bspline_sum(grows(u, A[0].base, A[1].base, A[2].base, n1, n2), A[0], A[1], A[2], m.inv_dx, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -323,7 +364,9 @@ EDGE_D float mac_sample_comp(const Mac& m, const float p[3], int a) {
 // coordinate is in (i - 1, i + 1.5) on each axis, i the thread's cell: tap
 // nodes floor(q - 0.5) .. + 2 and, staggered, floor(q - 1) .. + 2, and the
 // clamped ones near the walls (a cell index is at most n - 1).  A warp with a
-// sample outside that takes it from global memory.
+// sample outside that takes it from global memory.  A step of up to a cell, as
+// the CFL condition gives, stays inside; at four cells, which no driver takes,
+// the marches of 64x32x32 cost up to a tenth more than without a tile.
 // ---------------------------------------------------------------------------
 // Blocks of 4 x 4 x 8 cells: 2 x 2 x 32 stage more nodes per cell, were slower
 // and leave more of a ragged grid's threads idle.
@@ -434,7 +477,7 @@ EDGE_D void mac_sample(const MacTile<T>& t, const float p[3], float v[3], float 
         v[2] = bspline_sum(t.rows(2, A5[0].base, A5[1].base, A0[2].base), A5[0], A5[1], A0[2], t.m.inv_dx,
                            GRAD ? G[2] : nullptr);
     } else {
-        mac_sums<GRAD, false>(t.m, A0, A5, v, G);
+        mac_sums<GRAD>(t.m, A0, A5, v, G);
     }
 }
 

@@ -30,7 +30,7 @@ __global__ void k_lp_acc(Mac mac_, const float* __restrict__ vel, const float* _
         float kk = 1.0f / St;
         float p[3] = {pos[3 * e], pos[3 * e + 1], pos[3 * e + 2]};
         float v[3];
-        mac_sample<false, true>(mac, p, v, nullptr);
+        mac_sample_points(mac, p, v);
         a[1] += gravity;
         for (int c = 0; c < 3; c++) a[c] -= kk * (vel[3 * e + c] - v[c]);
         for (int c = 0; c < 3; c++) a[c] /= (1.0f + kk * dt);
@@ -63,7 +63,7 @@ __global__ void k_lp_vel_diff(Mac mac_, const float* __restrict__ vel, float* vd
     if (e >= num) return;
     float p[3] = {pos[3 * e], pos[3 * e + 1], pos[3 * e + 2]};
     float v[3];
-    mac_sample<false, true>(mac, p, v, nullptr);
+    mac_sample_points(mac, p, v);
     for (int c = 0; c < 3; c++) vdiff[3 * e + c] = kk * (vel[3 * e + c] - v[c]);
 }
 
