@@ -123,7 +123,8 @@ __constant__ float c_ed4_off[4][3] = {{-1, -1, -1}, {1, 1, -1}, {-1, 1, 1}, {1, 
 __constant__ float c_ed8_off[8][3] = {{-1, -1, -1}, {1, -1, -1}, {-1, 1, -1}, {1, 1, -1},   // hermite.py:716-723
                                       {-1, -1, 1},  {1, -1, 1},  {-1, 1, 1},  {1, 1, 1}};
 
-template <bool IDENT>
+// Reference layout, straight from the map: the ggg term of a corner comes from
+// its neighbours at every evaluation.
 __global__ void __launch_bounds__(128) k_march_edge(Mac mac, MapF m, float dt, float eps, float* __restrict__ opsi,
                                                     float* __restrict__ oTx, float* __restrict__ oTy,
                                                     float* __restrict__ oTz, float* __restrict__ odTx,
@@ -147,23 +148,12 @@ __global__ void __launch_bounds__(128) k_march_edge(Mac mac, MapF m, float dt, f
         }
         rk4_jac<3>(mac, P, C, -dt);
         float T[3][3];  // rows of the composed Jacobian
-        if (IDENT) {
-            // Hermite of the identity map reproduces the (clamped) position;
-            // its gradient is the identity.
-            for (int c = 0; c < 3; c++) {
-                float u = over_dx(P[c], m.dx, m.inv_dx, m.pow2) - 0.5f;
-                float s = fmaxf(1.0f, fminf(u, m.hi[c]));
-                P[c] = (s + 0.5f) * m.dx;
-                for (int d = 0; d < 3; d++) T[c][d] = C[d][c];
-            }
-        } else {
-            float val[3], G[3][3];
-            hermite3<HV_GARM, true>(m, P, val, G);
-            // T = T_old @ T_step, T_step rows: T_step[r][d] = C[d][r]
-            for (int r = 0; r < 3; r++)
-                for (int d = 0; d < 3; d++) T[r][d] = G[r][0] * C[d][0] + G[r][1] * C[d][1] + G[r][2] * C[d][2];
-            for (int c = 0; c < 3; c++) P[c] = val[c];
-        }
+        float val[3], G[3][3];
+        hermite3<HV_GARM, true>(m, P, val, G);
+        // T = T_old @ T_step, T_step rows: T_step[r][d] = C[d][r]
+        for (int r = 0; r < 3; r++)
+            for (int d = 0; d < 3; d++) T[r][d] = G[r][0] * C[d][0] + G[r][1] * C[d][1] + G[r][2] * C[d][2];
+        for (int c = 0; c < 3; c++) P[c] = val[c];
         if (q == 0) {
             for (int c = 0; c < 3; c++) {
                 Pc[c] = P[c];
@@ -214,6 +204,35 @@ EDGE_D void compose_jac(const float (&G)[3][3], const float (&C)[3][3], float (&
         }
 }
 
+// Where a march's results go, by packed plane: to a packed map, or to the
+// fields of the reference's layout.
+struct PlanesOut {
+    float4* __restrict__ g;
+    size_t n;
+    EDGE_D void put(int q, int e, float x, float y, float z) const { g[q * n + e] = make_float4(x, y, z, 0.f); }
+};
+struct Fields {
+    float* psi;
+    float* T[3];
+    float* dT[3];
+    EDGE_D void put(int q, int e, float x, float y, float z) const {
+        if (q == 0) {
+            psi[3 * e] = x; psi[3 * e + 1] = y; psi[3 * e + 2] = z;
+        } else {
+            float* const* f = q < 4 ? T : dT;
+            const int d = (q - 1) % 3;
+            f[0][3 * e + d] = x; f[1][3 * e + d] = y; f[2][3 * e + d] = z;
+        }
+    }
+};
+struct FieldsOut {
+    Fields to, map;  // map.psi null: only `to`
+    EDGE_D void put(int q, int e, float x, float y, float z) const {
+        to.put(q, e, x, y, z);
+        if (map.psi) map.put(q, e, x, y, z);
+    }
+};
+
 // The per-cell accumulators (the centre point's psi and Jacobian, the A and B
 // groups of the mixed derivatives) live in shared memory, one column per
 // thread, so that the registers hold only the current point's trajectory: four
@@ -223,9 +242,9 @@ EDGE_D void compose_jac(const float (&G)[3][3], const float (&C)[3][3], float (&
 // 61 us, from the identity 2026 -> 1600 us, with samples from the block's tile
 // and paired contractions.
 // mac: Mac, or MacTile where the block has staged its velocities.
-template <bool IDENT, bool F64, class M>
+template <bool IDENT, bool F64, class M, class Out>
 EDGE_D void march_edge_cell(const M& mac, const MapP& m, int i, int j, int k, float dt, float eps, float (&acc)[30][128],
-                            float4* __restrict__ out) {
+                            const Out& out) {
     float(&Pc)[3][128] = *reinterpret_cast<float(*)[3][128]>(&acc[0][0]);
     float(&Tc)[9][128] = *reinterpret_cast<float(*)[9][128]>(&acc[3][0]);
     float(&dA)[9][128] = *reinterpret_cast<float(*)[9][128]>(&acc[12][0]);
@@ -276,13 +295,12 @@ EDGE_D void march_edge_cell(const M& mac, const MapP& m, int i, int j, int k, fl
             }
         }
     }
-    out[e] = make_float4(Pc[0][tx], Pc[1][tx], Pc[2][tx], 0.f);
+    out.put(0, e, Pc[0][tx], Pc[1][tx], Pc[2][tx]);
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        out[(size_t)(1 + d) * n + e] = make_float4(Tc[d][tx], Tc[3 + d][tx], Tc[6 + d][tx], 0.f);
-        out[(size_t)(4 + d) * n + e] =
-            make_float4((dA[d][tx] + dB[d][tx]) / 8.0f / eps, (dA[3 + d][tx] + dB[3 + d][tx]) / 8.0f / eps,
-                        (dA[6 + d][tx] + dB[6 + d][tx]) / 8.0f / eps, 0.f);
+        out.put(1 + d, e, Tc[d][tx], Tc[3 + d][tx], Tc[6 + d][tx]);
+        out.put(4 + d, e, (dA[d][tx] + dB[d][tx]) / 8.0f / eps, (dA[3 + d][tx] + dB[3 + d][tx]) / 8.0f / eps,
+                (dA[6 + d][tx] + dB[6 + d][tx]) / 8.0f / eps);
     }
 }
 
@@ -303,8 +321,8 @@ EDGE_D void packed_cell(const Mac& mac_, const MapP& m, F f) {
     }
 }
 
-template <bool IDENT, bool F64, bool P2, class T>
-__global__ void __launch_bounds__(128, IDENT ? 5 : 4) k_march_edge_p(Mac mac, MapP m_, float dt, float eps, float4* __restrict__ out) {
+template <bool IDENT, bool F64, bool P2, class T, class Out>
+__global__ void __launch_bounds__(128, IDENT ? 5 : 4) k_march_edge_p(Mac mac, MapP m_, float dt, float eps, Out out) {
     const MapP m = with_pow2<P2>(m_);
     __shared__ float acc[30][128];
     packed_cell<T, P2>(mac, m, [&](const auto& smp, int i, int j, int k) {
@@ -314,11 +332,11 @@ __global__ void __launch_bounds__(128, IDENT ? 5 : 4) k_march_edge_p(Mac mac, Ma
 
 // ED4 march on the packed layout; output planes 0-3.  256x128x128: 1853 ->
 // 1647 us with samples from the tile.
-template <bool P2, class T>
-__global__ void __launch_bounds__(128) k_march_ed4_p(Mac mac_, MapP m_, float dt, float eps, float4* __restrict__ out) {
+template <bool P2, class T, class Out>
+__global__ void __launch_bounds__(128) k_march_ed4_p(Mac mac_, MapP m_, float dt, float eps, Out out) {
     const MapP m = with_pow2<P2>(m_);
     packed_cell<T, P2>(mac_, m, [&](const auto& mac, int i, int j, int k) {
-        const int n = m.n, e = idx3(i, j, k, m.ny, m.nz);
+        const int e = idx3(i, j, k, m.ny, m.nz);
         float X[3];
         cell_pos(i, j, k, m.dx, X);
         float P[4][3];
@@ -338,7 +356,8 @@ __global__ void __launch_bounds__(128) k_march_ed4_p(Mac mac_, MapP m_, float dt
             o[2][c] = (-P[0][c] + P[1][c] + P[2][c] - P[3][c]) / 4.0f / eps;
             o[3][c] = (-P[0][c] - P[1][c] + P[2][c] + P[3][c]) / 4.0f / eps;
         }
-        for (int q = 0; q < 4; q++) out[(size_t)q * n + e] = make_float4(o[q][0], o[q][1], o[q][2], 0.f);
+#pragma unroll
+        for (int q = 0; q < 4; q++) out.put(q, e, o[q][0], o[q][1], o[q][2]);
     });
 }
 
@@ -1288,6 +1307,32 @@ void with_tile(int nx, int ny, int nz, double fill, F f) {
     else f(NoTile{}, grid_for(n, 128));
 }
 
+template <class Out>
+void march_edge_by(const Mac& mac, const MapP& m, float dt, float eps, bool identity, bool f64, Out out,
+                   cudaStream_t st) {
+    with_tile(mac.nx, mac.ny, mac.nz, 0.9, [&](auto t, int g) {
+        using T = decltype(t);
+        auto launch = [&](auto k) { k<<<g, 128, 0, st>>>(mac, m, dt, eps, out); };
+        if (mac.pow2) {
+            if (identity) launch(k_march_edge_p<true, false, true, T, Out>);
+            else if (f64) launch(k_march_edge_p<false, true, true, T, Out>);
+            else launch(k_march_edge_p<false, false, true, T, Out>);
+        } else {
+            if (identity) launch(k_march_edge_p<true, false, false, T, Out>);
+            else if (f64) launch(k_march_edge_p<false, true, false, T, Out>);
+            else launch(k_march_edge_p<false, false, false, T, Out>);
+        }
+    });
+}
+template <class Out>
+void march_ed4_by(const Mac& mac, const MapP& m, float dt, float eps, Out out, cudaStream_t st) {
+    with_tile(mac.nx, mac.ny, mac.nz, 0.8, [&](auto t, int g) {
+        using T = decltype(t);
+        if (mac.pow2) k_march_ed4_p<true, T, Out><<<g, 128, 0, st>>>(mac, m, dt, eps, out);
+        else k_march_ed4_p<false, T, Out><<<g, 128, 0, st>>>(mac, m, dt, eps, out);
+    });
+}
+
 }  // namespace
 
 // ===========================================================================
@@ -1376,13 +1421,12 @@ int edge_march_edge(int nx, int ny, int nz, float dx, float dt, float epsilon, c
     const float* dT[3] = {dTx, dTy, dTz};
     MapF m = make_map(psi, T, dT, nullptr, nx, ny, nz, dx);
     Mac mac = make_mac(ux, uy, uz, nx, ny, nz, dx);
-    int n = nx * ny * nz;
-    if (identity)
-        k_march_edge<true><<<grid_for(n, 128), 128, 0, S(stream)>>>(mac, m, dt, epsilon, opsi, oTx, oTy, oTz, odTx,
-                                                                    odTy, odTz);
+    if (identity)  // the map is not read, its packed form need not exist
+        march_edge_by(mac, make_mapp(nullptr, nx, ny, nz, dx), dt, epsilon, true, false,
+                      FieldsOut{{opsi, {oTx, oTy, oTz}, {odTx, odTy, odTz}}, {}}, S(stream));
     else
-        k_march_edge<false><<<grid_for(n, 128), 128, 0, S(stream)>>>(mac, m, dt, epsilon, opsi, oTx, oTy, oTz, odTx,
-                                                                     odTy, odTz);
+        k_march_edge<<<grid_for(nx * ny * nz, 128), 128, 0, S(stream)>>>(mac, m, dt, epsilon, opsi, oTx, oTy, oTz,
+                                                                         odTx, odTy, odTz);
     return launch_status();
 }
 
@@ -1524,26 +1568,37 @@ int edge_march_packed(int variant, int nx, int ny, int nz, float dx, float dt, f
     MapP m = make_mapp(in_packed, nx, ny, nz, dx);
     Mac mac = make_mac(ux, uy, uz, nx, ny, nz, dx);
     float4* o = (float4*)out_packed;
-    with_tile(nx, ny, nz, variant == HV_GARM ? 0.9 : 0.8, [&](auto t, int g) {
-        using T = decltype(t);
-        auto launch = [&](auto k) { k<<<g, 128, 0, S(stream)>>>(mac, m, dt, epsilon, o); };
-        if (variant == HV_GARM && mac.pow2) {
-            if (identity) launch(k_march_edge_p<true, false, true, T>);
-            else if (f64) launch(k_march_edge_p<false, true, true, T>);
-            else launch(k_march_edge_p<false, false, true, T>);
-        } else if (variant == HV_GARM) {
-            if (identity) launch(k_march_edge_p<true, false, false, T>);
-            else if (f64) launch(k_march_edge_p<false, true, false, T>);
-            else launch(k_march_edge_p<false, false, false, T>);
-        } else if (variant == HV_FD) {
-            if (mac.pow2) launch(k_march_ed4_p<true, T>);
-            else launch(k_march_ed4_p<false, T>);
-        } else {
-            if (mac.pow2) launch(k_march_ed8_p<true, T>);
-            else launch(k_march_ed8_p<false, T>);
-        }
-    });
+    if (variant == HV_GARM) march_edge_by(mac, m, dt, epsilon, identity, f64, PlanesOut{o, (size_t)m.n}, S(stream));
+    else if (variant == HV_FD) march_ed4_by(mac, m, dt, epsilon, PlanesOut{o, (size_t)m.n}, S(stream));
+    else
+        with_tile(nx, ny, nz, 0.8, [&](auto t, int g) {
+            using T = decltype(t);
+            if (mac.pow2) k_march_ed8_p<true, T><<<g, 128, 0, S(stream)>>>(mac, m, dt, epsilon, o);
+            else k_march_ed8_p<false, T><<<g, 128, 0, S(stream)>>>(mac, m, dt, epsilon, o);
+        });
     derive_planes(variant, nx, ny, nz, out_packed, S(stream));
+    return launch_status();
+}
+
+int edge_march_fields(int variant, int nx, int ny, int nz, float dx, float dt, float epsilon, const float* ux,
+                      const float* uy, const float* uz, float* psi, float* Tx, float* Ty, float* Tz, float* dTx,
+                      float* dTy, float* dTz, float* opsi, float* oTx, float* oTy, float* oTz, float* odTx,
+                      float* odTy, float* odTz, int update, float* work, void* stream) {
+    const bool edge = variant == HV_GARM;
+    if ((!edge && variant != HV_FD) || !dims_ok(nx, ny, nz) || !ux || !uy || !uz || !psi || !Tx || !Ty || !Tz ||
+        !opsi || !oTx || !oTy || !oTz || !work)
+        return EDGE_EINVAL;
+    if (edge && (!dTx || !dTy || !dTz || !odTx || !odTy || !odTz || odTx == dTx)) return EDGE_EINVAL;
+    if (opsi == psi || oTx == Tx || (!edge && (oTy == Ty || oTz == Tz))) return EDGE_EINVAL;
+    const int rc = edge_map_pack(variant, nx, ny, nz, psi, Tx, Ty, Tz, dTx, dTy, dTz, nullptr, nullptr, nullptr, work,
+                                 stream);
+    if (rc != EDGE_OK) return rc;
+    const MapP m = make_mapp(work, nx, ny, nz, dx);
+    const Mac mac = make_mac(ux, uy, uz, nx, ny, nz, dx);
+    FieldsOut out{{opsi, {oTx, oTy, oTz}, {odTx, odTy, odTz}}, {}};
+    if (update) out.map = Fields{psi, {Tx, Ty, Tz}, {dTx, dTy, dTz}};
+    if (edge) march_edge_by(mac, m, dt, epsilon, false, false, out, S(stream));
+    else march_ed4_by(mac, m, dt, epsilon, out, S(stream));
     return launch_status();
 }
 

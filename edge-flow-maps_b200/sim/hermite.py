@@ -31,22 +31,18 @@ _ED8_OFF = ((-1, -1, -1), (1, -1, -1), (-1, 1, -1), (1, 1, -1),                 
 
 def advect_psi_garm_ed4_fusion_unroll(psi_tmp, T_x_tmp, T_y_tmp, T_z_tmp, dT_x_tmp, dT_y_tmp, dT_z_tmp,
                                       psi, T_x, T_y, T_z, dT_x, dT_y, dT_z, u_x, u_y, u_z, X, dx, dt, epsilon):
-    """hermite.py:1495-1521: EDGE march into the *_tmp fields, then copied
-    into the accumulated map."""
+    """hermite.py:1495-1521: EDGE march into the *_tmp fields and the
+    accumulated map."""
     ops.march_edge((u_x, u_y, u_z), dx, dt, epsilon, psi, (T_x, T_y, T_z), (dT_x, dT_y, dT_z), psi_tmp,
-                   (T_x_tmp, T_y_tmp, T_z_tmp), (dT_x_tmp, dT_y_tmp, dT_z_tmp))
-    for d, s in ((psi, psi_tmp), (T_x, T_x_tmp), (T_y, T_y_tmp), (T_z, T_z_tmp), (dT_x, dT_x_tmp),
-                 (dT_y, dT_y_tmp), (dT_z, dT_z_tmp)):
-        ops.copy(s, d)
+                   (T_x_tmp, T_y_tmp, T_z_tmp), (dT_x_tmp, dT_y_tmp, dT_z_tmp), update=True)
 
 
 def advect_ps_hermite_ed4_fd_unroll(psi_0, psi_1, psi_2, psi_3, psi, T_x, T_y, T_z, u_x, u_y, u_z, X, dx, dt,
                                     epsilon):
     """hermite.py:1375-1395: ED4 march (the four scratch fields receive the new
-    psi, T_x, T_y, T_z before the copy back)."""
-    ops.march_ed4((u_x, u_y, u_z), dx, dt, epsilon, psi, (T_x, T_y, T_z), psi_0, (psi_1, psi_2, psi_3))
-    for d, s in ((psi, psi_0), (T_x, psi_1), (T_y, psi_2), (T_z, psi_3)):
-        ops.copy(s, d)
+    psi, T_x, T_y, T_z as well)."""
+    ops.march_ed4((u_x, u_y, u_z), dx, dt, epsilon, psi, (T_x, T_y, T_z), psi_0, (psi_1, psi_2, psi_3),
+                  update=True)
 
 
 def advect_ps_hermite_ed8(psi_000, psi_001, psi_010, psi_011, psi_100, psi_101, psi_110, psi_111,

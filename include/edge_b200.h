@@ -153,6 +153,17 @@ int edge_map_unpack(int variant, int nx, int ny, int nz, const float *packed, fl
 int edge_march_packed(int variant, int nx, int ny, int nz, float dx, float dt, float epsilon, const float *ux,
                       const float *uy, const float *uz, const float *in_packed, float *out_packed, int flags,
                       void *stream);
+/* edge_march_edge (variant 1) and edge_march_ed4 (variant 0, whose dT and odT
+ * may be null) through a packed copy of the map: the same results, with the
+ * Hermite terms that the reference derives by finite differences formed once
+ * per cell instead of at every evaluation.  work: one packed map
+ * (edge_packed_planes x cells float4, 16-byte aligned), free again when the
+ * call's work on the stream is done.  The outputs must not alias the inputs;
+ * if `update` is non-zero psi, T and dT receive the results as well. */
+int edge_march_fields(int variant, int nx, int ny, int nz, float dx, float dt, float epsilon, const float *ux,
+                      const float *uy, const float *uz, float *psi, float *Tx, float *Ty, float *Tz, float *dTx,
+                      float *dTy, float *dTz, float *opsi, float *oTx, float *oTy, float *oTz, float *odTx,
+                      float *odTy, float *odTz, int update, float *work, void *stream);
 /* edge_march_ge on packed maps (the ED8 planes 0-7); out_packed must not
  * alias in_packed. */
 int edge_march_ge_packed(int nx, int ny, int nz, float dx, float dt, const float *ux, const float *uy,

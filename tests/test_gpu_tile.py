@@ -1,7 +1,8 @@
 """Marches and semi-Lagrangian advection by tiles of cells, whose velocity
 samples come from shared memory (or, from a warp with a sample outside the
-tile, from global memory): the marches against the reference-layout ones, which
-always read global memory, the advection against the oracle."""
+tile, from global memory): the marches, of packed maps and of fields through a
+packed copy, against the ones straight from the fields, which always read
+global memory, the advection against the oracle."""
 import numpy as np
 import pytest
 
@@ -15,7 +16,7 @@ torch = pytest.importorskip("torch")
                                     ((15, 16, 24), 1 / 16), ((16, 15, 23), 1 / 23), ((9, 17, 33), 1 / 32)])
 @pytest.mark.parametrize("cells", [0.3, 3.0])
 @pytest.mark.parametrize("variant", [0, 1, 2, "identity"])
-def test_march_by_tiles(res, dx, cells, variant):
+def test_march_by_tiles(res, dx, cells, variant, monkeypatch):
     from edgeb200 import ops
     from edgeb200.fields import zeros_faces
     identity, variant = variant == "identity", 1 if variant == "identity" else variant
@@ -38,8 +39,17 @@ def test_march_by_tiles(res, dx, cells, variant):
     out = torch.full_like(packed, float("nan"))
     ops.map_pack(variant, psi, T, dT, d2T, packed)
     ops.march_packed(variant, u, dx, dt, eps, packed, out, res, identity=identity)
+    f = [vec() for _ in range(7)]
+    state = [t.clone() for t in [psi, *T, *(dT or [])]]
     if variant == 1:
-        ops.march_edge(u, dx, dt, eps, psi, T, dT, o[0], o[1:4], o[4:7], identity=identity)
+        ops.march_edge(u, dx, dt, eps, state[0], state[1:4], state[4:7], f[0], f[1:4], f[4:7], identity=identity,
+                       update=True)
+    elif variant == 0:
+        ops.march_ed4(u, dx, dt, eps, state[0], state[1:4], f[0], f[1:4], update=True)
+    # straight from the fields; the identity map as any other
+    monkeypatch.setattr(ops, "_map_workspace", lambda psi: None)
+    if variant == 1:
+        ops.march_edge(u, dx, dt, eps, psi, T, dT, o[0], o[1:4], o[4:7])
     elif variant == 0:
         ops.march_ed4(u, dx, dt, eps, psi, T, o[0], o[1:4])
     else:
@@ -52,12 +62,15 @@ def test_march_by_tiles(res, dx, cells, variant):
     s = 2 * cells
     tol = 4 * ulp * 2 * (1 + s + s**2 / 2 + s**3 / 4 + s**4 / 24)
     tol_T = tol / eps if variant != 1 else 8 * tol / dx
-    assert float((q[0] - o[0]).abs().max()) <= 4 * tol
-    for a, b in zip(q[1:4], o[1:4]):
-        assert float((a - b).abs().max()) <= tol_T * (1 + s)**3
-    for a, b in zip(q[4:7], o[4:7]):
-        if variant:
-            assert float((a - b).abs().max()) <= tol_T * (1 + s)**3 / eps
+    for r in [q] if variant == 2 else [q, f]:
+        assert float((r[0] - o[0]).abs().max()) <= 4 * tol
+        for a, b in zip(r[1:4], o[1:4]):
+            assert float((a - b).abs().max()) <= tol_T * (1 + s)**3
+        for a, b in zip(r[4:7], o[4:7]):
+            if variant:
+                assert float((a - b).abs().max()) <= tol_T * (1 + s)**3 / eps
+    if variant != 2:
+        assert all(torch.equal(a, b) for a, b in zip(state, f))
 
 
 # the smallest grids that take tiles, a ragged one and one just below
