@@ -616,17 +616,6 @@ __global__ void k_coef_p(MapP m, float4* __restrict__ g) {
 // 256x128x128: 818 us for one 64-coefficient launch per axis, 111 us so (the
 // copy bandwidth allows 90); 192x96x96, where a quarter of the faces is left
 // over: 363 and 218 us.
-struct Face3 {
-    const float* p[3];
-    // select with constant indices only: a run-time index into a kernel
-    // parameter array makes the compiler copy the parameter to local memory
-    EDGE_D const float* at(int a) const { return a == 0 ? p[0] : (a == 1 ? p[1] : p[2]); }
-};
-struct Face3W {
-    float* p[3];
-    EDGE_D float* at(int a) const { return a == 0 ? p[0] : (a == 1 ? p[1] : p[2]); }
-};
-
 // Hermite coordinate of axis d's cell centre i as hermite3p forms it: its base
 // cell, and whether it has no fractional part
 struct Centre {
@@ -1086,22 +1075,13 @@ __global__ void __launch_bounds__(128) k_smoke_psi(Dye dye, MapF m, const float*
 }
 
 // clamp_u (run_edge.py:509-519) over the three face grids
-__global__ void k_clamp_u(int nx, int ny, int nz, Face3 u, Face3 u1, float* ox, float* oy, float* oz) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_faces(nx, ny, nz)) return;
-    FaceIdx f = face_decompose(t, nx, ny, nz);
-    int n0 = nx + (f.axis == 0), n1 = ny + (f.axis == 1), n2 = nz + (f.axis == 2);
-    const float* a = u1.at(f.axis);
-    int im = max(f.i - 1, 0), ip = min(f.i + 1, n0 - 1);
-    int jm = max(f.j - 1, 0), jp = min(f.j + 1, n1 - 1);
-    int km = max(f.k - 1, 0), kp = min(f.k + 1, n2 - 1);
-    float l = __ldg(a + idx3(im, f.j, f.k, n1, n2)), r = __ldg(a + idx3(ip, f.j, f.k, n1, n2));
-    float b = __ldg(a + idx3(f.i, jm, f.k, n1, n2)), tt = __ldg(a + idx3(f.i, jp, f.k, n1, n2));
-    float aa = __ldg(a + idx3(f.i, f.j, km, n1, n2)), cc = __ldg(a + idx3(f.i, f.j, kp, n1, n2));
-    float mx = fmaxf(fmaxf(fmaxf(fmaxf(fmaxf(l, r), b), tt), aa), cc);
-    float mn = fminf(fminf(fminf(fminf(fminf(l, r), b), tt), aa), cc);
-    float* o = f.axis == 0 ? ox : (f.axis == 1 ? oy : oz);
-    o[f.e] = fminf(fmaxf(__ldg(u.at(f.axis) + f.e), mn), mx);
+__global__ void __launch_bounds__(256) k_clamp_u(Star g, Face3 u, Face3 u1, float* ox, float* oy, float* oz) {
+    face_star(g, u1, [&](int axis, int e, float, float l, float r, float b, float t, float a, float c) {
+        const float mx = fmaxf(fmaxf(fmaxf(fmaxf(fmaxf(l, r), b), t), a), c);
+        const float mn = fminf(fminf(fminf(fminf(fminf(l, r), b), t), a), c);
+        float* o = axis == 0 ? ox : (axis == 1 ? oy : oz);
+        o[e] = fminf(fmaxf(__ldg(u.at(axis) + e), mn), mx);
+    });
 }
 
 __global__ void k_set_float(float* p, float v) { *p = v; }
@@ -1800,7 +1780,8 @@ int edge_clamp_u(int nx, int ny, int nz, const float* ux, const float* uy, const
     if (!dims_ok(nx, ny, nz) || !ux || !uy || !uz || !u1x || !u1y || !u1z || !u2x || !u2y || !u2z) return EDGE_EINVAL;
     if (u2x == u1x || u2y == u1y || u2z == u1z) return EDGE_EINVAL;
     Face3 u = {{ux, uy, uz}}, u1 = {{u1x, u1y, u1z}};
-    k_clamp_u<<<grid_for(n_faces(nx, ny, nz)), kBlock, 0, S(stream)>>>(nx, ny, nz, u, u1, u2x, u2y, u2z);
+    const Star g = make_star(nx, ny, nz);
+    k_clamp_u<<<star_grid(g, 256), 256, 0, S(stream)>>>(g, u, u1, u2x, u2y, u2z);
     return launch_status();
 }
 

@@ -1164,4 +1164,61 @@ EDGE_HD long long n_faces(int nx, int ny, int nz) {
     return (long long)(nx + 1) * ny * nz + (long long)nx * (ny + 1) * nz + (long long)nx * ny * (nz + 1);
 }
 
+struct Face3 {
+    const float* p[3];
+    // select with constant indices only: a run-time index into a kernel
+    // parameter array makes the compiler copy the parameter to local memory
+    EDGE_D const float* at(int a) const { return a == 0 ? p[0] : (a == 1 ? p[1] : p[2]); }
+};
+struct Face3W {
+    float* p[3];
+    EDGE_D float* at(int a) const { return a == 0 ? p[0] : (a == 1 ? p[1] : p[2]); }
+};
+
+// ---------------------------------------------------------------------------
+// Seven-point stencils over the three face grids (blockIdx.y: the component),
+// neighbours clamped to the grid.  A thread takes one (j, k) of `chunk`
+// consecutive i's: one division for all of them, and the i neighbours stay in
+// registers, five loads a face instead of seven.  Bound by memory.  256x128x128,
+// one face per thread and so: clamp 76 -> 43 us, viscous force 83 -> 35 us.
+// f(axis, e, centre, low and high neighbour of x, of y, of z).
+// ---------------------------------------------------------------------------
+struct Star {
+    int nx, ny, nz, chunk;
+};
+template <class F>
+EDGE_D void face_star(const Star& g, const Face3& field, F f) {
+    const int axis = blockIdx.y;
+    const int n0 = g.nx + (axis == 0), n1 = g.ny + (axis == 1), n2 = g.nz + (axis == 2), plane = n1 * n2;
+    const float* __restrict__ a = field.at(axis);
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, c = t / (unsigned)plane;
+    const int m = (int)(t - c * (unsigned)plane), i0 = (int)c * g.chunk, i1 = min(i0 + g.chunk, n0);
+    if (i0 >= n0) return;
+    const unsigned j = (unsigned)m / (unsigned)n2, k = (unsigned)m - j * (unsigned)n2;
+    const int jl = j > 0 ? -n2 : 0, jh = (int)j < n1 - 1 ? n2 : 0, kl = k > 0 ? -1 : 0, kh = (int)k < n2 - 1;
+    int e = i0 * plane + m;
+    float lo = __ldg(a + (i0 > 0 ? e - plane : e)), at = __ldg(a + e);
+#pragma unroll 4
+    for (int i = i0; i < i1; i++, e += plane) {
+        const float hi = i < n0 - 1 ? __ldg(a + e + plane) : at;
+        f(axis, e, at, lo, hi, __ldg(a + e + jl), __ldg(a + e + jh), __ldg(a + e + kl), __ldg(a + e + kh));
+        lo = at;
+        at = hi;
+    }
+}
+// up to eight faces a thread while that leaves a full wave of threads
+static inline Star make_star(int nx, int ny, int nz) {
+    const long long n = n_faces(nx, ny, nz) / (148LL * 2048);
+    return Star{nx, ny, nz, (int)(n < 1 ? 1 : (n > 8 ? 8 : n))};
+}
+static inline dim3 star_grid(const Star& s, int block) {
+    long long most = 0;
+    for (int a = 0; a < 3; a++) {
+        const long long n0 = s.nx + (a == 0), n1 = s.ny + (a == 1), n2 = s.nz + (a == 2);
+        const long long n = (n0 + s.chunk - 1) / s.chunk * n1 * n2;
+        if (n > most) most = n;
+    }
+    return dim3((unsigned)((most + block - 1) / block), 3);
+}
+
 }  // namespace edge

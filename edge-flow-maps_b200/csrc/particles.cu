@@ -333,21 +333,14 @@ __global__ void k_lp_position(const float* __restrict__ vel, float* pos, float d
 }
 
 // lp.py:183-219 calculate_viscous_force on the three face grids
-__global__ void k_lp_viscous(int nx, int ny, int nz, float dx, float nu, const float* __restrict__ ux,
-                             const float* __restrict__ uy, const float* __restrict__ uz, float* vx, float* vy,
-                             float* vz) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_faces(nx, ny, nz)) return;
-    FaceIdx f = face_decompose(t, nx, ny, nz);
-    int n0 = nx + (f.axis == 0), n1 = ny + (f.axis == 1), n2 = nz + (f.axis == 2);
-    const float* u = f.axis == 0 ? ux : (f.axis == 1 ? uy : uz);
-    float* o = f.axis == 0 ? vx : (f.axis == 1 ? vy : vz);
-    auto s = [&](int i, int j, int k) {
-        return __ldg(u + idx3(min(max(i, 0), n0 - 1), min(max(j, 0), n1 - 1), min(max(k, 0), n2 - 1), n1, n2));
-    };
-    int i = f.i, j = f.j, k = f.k;
-    o[f.e] = nu * (s(i + 1, j, k) + s(i - 1, j, k) + s(i, j + 1, k) + s(i, j - 1, k) + s(i, j, k + 1) +
-                   s(i, j, k - 1) + -6.0f * s(i, j, k)) / dx / dx;
+template <bool P2>
+__global__ void __launch_bounds__(256) k_lp_viscous(Star g, float dx, float inv_dx, float nu, Face3 u, float* vx,
+                                                    float* vy, float* vz) {
+    face_star(g, u, [&](int axis, int e, float at, float l, float r, float b, float t, float a, float c) {
+        float* o = axis == 0 ? vx : (axis == 1 ? vy : vz);
+        const float v = nu * (r + l + t + b + c + a + -6.0f * at);
+        o[e] = over_dx(over_dx(v, dx, inv_dx, P2), dx, inv_dx, P2);
+    });
 }
 
 // calc_max_particle_speed (run_edge.py:256-261): max |v| over the live
@@ -491,8 +484,11 @@ int edge_lp_position(const float* vel, float* pos, float dt, int num, float Lx, 
 int edge_lp_viscous(int nx, int ny, int nz, float dx, float Re, const float* ux, const float* uy, const float* uz,
                     float* visx, float* visy, float* visz, void* stream) {
     if (nx < 1 || ny < 1 || nz < 1 || !ux || !uy || !uz || !visx || !visy || !visz) return EDGE_EINVAL;
-    k_lp_viscous<<<grid_for(n_faces(nx, ny, nz)), 256, 0, S(stream)>>>(nx, ny, nz, dx, 1.0f / Re, ux, uy, uz, visx,
-                                                                       visy, visz);
+    const Star g = make_star(nx, ny, nz);
+    const Face3 u = {{ux, uy, uz}};
+    const float inv = 1.0f / dx, nu = 1.0f / Re;
+    if (pow2f(dx)) k_lp_viscous<true><<<star_grid(g, 256), 256, 0, S(stream)>>>(g, dx, inv, nu, u, visx, visy, visz);
+    else k_lp_viscous<false><<<star_grid(g, 256), 256, 0, S(stream)>>>(g, dx, inv, nu, u, visx, visy, visz);
     return st();
 }
 
