@@ -249,7 +249,7 @@ EDGE_D void march_edge_cell(const M& mac, const MapP& m, int i, int j, int k, fl
     float(&Tc)[9][128] = *reinterpret_cast<float(*)[9][128]>(&acc[3][0]);
     float(&dA)[9][128] = *reinterpret_cast<float(*)[9][128]>(&acc[12][0]);
     float(&dB)[9][128] = *reinterpret_cast<float(*)[9][128]>(&acc[21][0]);
-    const int tx = threadIdx.x, n = m.n, e = idx3(i, j, k, m.ny, m.nz);
+    const int tx = threadIdx.x, e = idx3(i, j, k, m.ny, m.nz);
     float X[3];
     cell_pos(i, j, k, m.dx, X);
 #pragma unroll 1
@@ -836,9 +836,10 @@ __global__ void __launch_bounds__(128) k_face_map(MapF m, float* fpx, float* fpy
     }
 }
 
-// advance_map x3 (run_edge.py:330-357)
+// advance_map x3 (run_edge.py:330-357).  Six blocks per SM: 256x128x128 1118 us
+// uncapped, 1090 at six, 1133 at eight.
 template <bool P2>
-__global__ void __launch_bounds__(128) k_advance_map(Mac mac_, float dt, float* phix, float* phiy, float* phiz,
+__global__ void __launch_bounds__(128, 6) k_advance_map(Mac mac_, float dt, float* phix, float* phiy, float* phiz,
                                                      float* Fx, float* Fy, float* Fz) {
     const Mac mac = with_pow2<P2>(mac_);
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -963,9 +964,12 @@ __global__ void __launch_bounds__(T::threads) k_advect_tile(Mac mac_, float dt, 
     }
 }
 
-// map_u / map_u_psi pullback with fused BFECC arithmetic (edge_pullback_u)
+// map_u / map_u_psi pullback with fused BFECC arithmetic (edge_pullback_u).
+// Waits for its gathers, so more warps are worth a few spills: 256x128x128
+// 318 us uncapped, 287 at six blocks per SM; with the divisions of a spacing
+// that is no power of two five (192x96x96 127 and 126 us, 130 at six).
 template <bool P2>
-__global__ void __launch_bounds__(256) k_pullback_u(Mac mac_, Face3 pos, Face3 col, Face3 init, float scale, Face3 sub,
+__global__ void __launch_bounds__(256, P2 ? 6 : 5) k_pullback_u(Mac mac_, Face3 pos, Face3 col, Face3 init, float scale, Face3 sub,
                                                     float* ox, float* oy, float* oz) {
     const Mac mac = with_pow2<P2>(mac_);
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
