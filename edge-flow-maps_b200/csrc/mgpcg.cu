@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <cmath>
 #include <cstddef>
 #include <cstdio>
@@ -523,41 +524,55 @@ __global__ void k_apply_solid(SolveState* st, int nx, int ny, int nz, const int*
 // mgpcg.py:394-404 divergence + init(u_div, -1) (mgpcg.py:67-75); solid:
 // mgpcg_solid.py:359-372 (fluid-only divergence, its sum and count).  With
 // rhs != NULL the right-hand side is taken from rhs instead (edge_mgpcg_solve).
-// One thread per slot handles the cell pair k = 2kk (plane (i+j)&1) and
-// k = 2kk+1 (the other plane).  x and p need no initialisation: the first
-// iteration writes them without reading them.
-template <bool SOLID>
+// x and p need no initialisation: the first iteration writes them without
+// reading them.
+//
+// This and k_grad_p walk lines along x in groups of kLine cells: the loads of
+// a group are issued together, a face between two of its cells is read once,
+// and one index decomposition serves the group.  Bound by memory: gradient
+// update 256x128x128 45 -> 32 us (two cells of a slot at a time, their stores
+// between the loads), a solve of 512x256x256 5116 -> 5000 us.
+template <bool SOLID, int kLine>
 __global__ void __launch_bounds__(256) k_setup_rhs(G g, Lvl L, Fine f, Faces U, const float* rhs, double abs_tol,
                                                    double rel_tol, int max_iters) {
     count_launch(g.st);
-    const int ny = L.n1, nz = L.n2;
+    const int nx = L.n0, ny = L.n1, nz = L.n2, plane = ny * nz, groups = (nx + kLine - 1) / kLine;
     double v[4] = {0.0, 0.0, 0.0, 0.0};  // sum div (fluid), fluid count, sum r, sum r^2
-    GRID_STRIDE(t, L.P) {
-        Slot s = slot_of(L, t);
-        const int c0 = (s.i + s.j) & 1;
+    GRID_STRIDE(t, plane * groups) {
+        const int q = t / plane, m = t - q * plane, i0 = q * kLine, j = m / nz, k = m - j * nz;
+        float d[kLine];
+        bool fl[kLine];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int k = 2 * s.kk + h;
-            if (k >= nz) break;
-            const int e = idx3(s.i, s.j, k, ny, nz);
-            const bool fl = !SOLID || L.bm[e] <= 0;
-            float d;
-            if (rhs) {
-                d = -rhs[e];
-            } else if (fl) {
-                const int i = s.i, j = s.j;
-                float vl = U.u[0][idx3(i, j, k, ny, nz)], vr = U.u[0][idx3(i + 1, j, k, ny, nz)];
-                float vb = U.u[1][idx3(i, j, k, ny + 1, nz)], vt = U.u[1][idx3(i, j + 1, k, ny + 1, nz)];
-                float va = U.u[2][idx3(i, j, k, ny, nz + 1)], vc = U.u[2][idx3(i, j, k + 1, ny, nz + 1)];
-                d = vr - vl + vt - vb + vc - va;
-            } else {
-                d = 0.0f;
+        for (int h = 0; h < kLine; h++) fl[h] = !SOLID || (i0 + h < nx && L.bm[(i0 + h) * plane + m] <= 0);
+        if (rhs) {
+#pragma unroll
+            for (int h = 0; h < kLine; h++) d[h] = i0 + h < nx ? -rhs[(i0 + h) * plane + m] : 0.0f;
+        } else {
+            float ux[kLine + 1], vb[kLine], vt[kLine], va[kLine], vc[kLine];
+#pragma unroll
+            for (int h = 0; h <= kLine; h++)
+                if (i0 + h <= nx) ux[h] = U.u[0][(i0 + h) * plane + m];
+#pragma unroll
+            for (int h = 0; h < kLine; h++) {
+                if (i0 + h >= nx) continue;
+                const float* y = U.u[1] + idx3(i0 + h, j, k, ny + 1, nz);
+                const float* z = U.u[2] + idx3(i0 + h, j, k, ny, nz + 1);
+                vb[h] = y[0]; vt[h] = y[nz];
+                va[h] = z[0]; vc[h] = z[1];
             }
-            f.div[e] = d;
-            float r = d * -1.0f;
-            pick(L.r, c0 ^ h)[t] = r;
-            if (fl) {
-                v[0] += d;
+#pragma unroll
+            for (int h = 0; h < kLine; h++)
+                d[h] = fl[h] ? ux[h + 1] - ux[h] + vt[h] - vb[h] + vc[h] - va[h] : 0.0f;
+        }
+#pragma unroll
+        for (int h = 0; h < kLine; h++) {
+            const int i = i0 + h;
+            if (i >= nx) break;
+            f.div[i * plane + m] = d[h];
+            const float r = d[h] * -1.0f;
+            pick(L.r, (i + j + k) & 1)[(i * ny + j) * L.H + (k >> 1)] = r;
+            if (fl[h]) {
+                v[0] += d[h];
                 v[1] += 1.0;
             }
             v[2] += r;
@@ -1806,39 +1821,50 @@ __global__ void __launch_bounds__(256) k_restrict4(G g, Lvl F, Lvl C, int level0
 
 // mgpcg.py:406-432 subtract_grad_p (p = x, get_result mgpcg.py:77-85) + the
 // wall part of the final apply_bc; Poisson_with_buffer's force (mgpcg.py:448-479).
-// One thread per slot: the faces on the low side of its two cells in each
-// axis, and the high boundary faces of cells on the high boundary.
-EDGE_D void face_update(const G& g, const Faces& U, int a, int e, float gr, bool at_wall) {
-    float* ua = pick3(U.u, a);
+// A cell updates the faces on its low sides, the last one of an axis the
+// boundary face as well.  ua: the face's velocity, loaded ahead of the stores.
+EDGE_D void face_update(const G& g, const Faces& U, int a, int e, float ua, float gr, bool at_wall) {
     float* fa = pick3(U.f, a);
-    float u = ua[e] - gr;
-    if (at_wall) u = 0.0f;
-    ua[e] = u;
+    pick3(U.u, a)[e] = at_wall ? 0.0f : ua - gr;
     if (fa) fa[e] = -gr;
 }
 
+template <int kLine>
 __global__ void __launch_bounds__(256) k_grad_p(G g, Lvl L, Fine f, Faces U) {
     count_launch(g.st);
     const bool xv = g.st->x_valid != 0;  // x = 0 when no iteration ran
-    const int nx = L.n0, ny = L.n1, nz = L.n2, sx = L.n1 * L.H;
-    GRID_STRIDE(t, L.P) {
-        const Slot s = slot_of(L, t);
-        const int i = s.i, j = s.j, c0 = (i + j) & 1;
+    const int nx = L.n0, ny = L.n1, nz = L.n2, plane = ny * nz, groups = (nx + kLine - 1) / kLine;
+    GRID_STRIDE(t, plane * groups) {
+        const int q = t / plane, m = t - q * plane, i0 = q * kLine, j = m / nz, k = m - j * nz;
+        auto x = [&](int i, int jj, int kk) {
+            return pick(f.x, (i + jj + kk) & 1)[(i * ny + jj) * L.H + (kk >> 1)];
+        };
+        float xc[kLine + 1], xy[kLine], xz[kLine], ux[kLine], uy[kLine], uz[kLine];
+        xc[0] = xv && i0 > 0 ? x(i0 - 1, j, k) : 0.0f;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int k = 2 * s.kk + h, pl = c0 ^ h;
-            if (k >= nz) break;
-            const float* xo = pick(f.x, pl ^ 1);
-            const float xc = xv ? pick(f.x, pl)[t] : 0.0f;
-            const float xl = (xv && i > 0) ? xo[t - sx] : 0.0f;
-            face_update(g, U, 0, idx3(i, j, k, ny, nz), xc - xl, i == 0 && wall(g.walls, 0));
-            if (i == nx - 1) face_update(g, U, 0, idx3(nx, j, k, ny, nz), 0.0f - xc, wall(g.walls, 1));
-            const float yl = (xv && j > 0) ? xo[t - L.H] : 0.0f;
-            face_update(g, U, 1, idx3(i, j, k, ny + 1, nz), xc - yl, j == 0 && wall(g.walls, 2));
-            if (j == ny - 1) face_update(g, U, 1, idx3(i, ny, k, ny + 1, nz), 0.0f - xc, wall(g.walls, 3));
-            const float zl = (xv && k > 0) ? xo[t - 1 + (k & 1)] : 0.0f;
-            face_update(g, U, 2, idx3(i, j, k, ny, nz + 1), xc - zl, k == 0 && wall(g.walls, 4));
-            if (k == nz - 1) face_update(g, U, 2, idx3(i, j, nz, ny, nz + 1), 0.0f - xc, wall(g.walls, 5));
+        for (int h = 0; h < kLine; h++) {
+            const int i = i0 + h;
+            const bool in = i < nx;
+            xc[h + 1] = xv && in ? x(i, j, k) : 0.0f;
+            xy[h] = xv && in && j > 0 ? x(i, j - 1, k) : 0.0f;
+            xz[h] = xv && in && k > 0 ? x(i, j, k - 1) : 0.0f;
+            if (!in) continue;
+            ux[h] = U.u[0][i * plane + m];
+            uy[h] = U.u[1][idx3(i, j, k, ny + 1, nz)];
+            uz[h] = U.u[2][idx3(i, j, k, ny, nz + 1)];
+        }
+#pragma unroll
+        for (int h = 0; h < kLine; h++) {
+            const int i = i0 + h;
+            if (i >= nx) break;
+            const float c = xc[h + 1];
+            face_update(g, U, 0, i * plane + m, ux[h], c - xc[h], i == 0 && wall(g.walls, 0));
+            face_update(g, U, 1, idx3(i, j, k, ny + 1, nz), uy[h], c - xy[h], j == 0 && wall(g.walls, 2));
+            face_update(g, U, 2, idx3(i, j, k, ny, nz + 1), uz[h], c - xz[h], k == 0 && wall(g.walls, 4));
+            auto high = [&](int a, int e, int b) { face_update(g, U, a, e, pick3(U.u, a)[e], 0.0f - c, wall(g.walls, b)); };
+            if (i == nx - 1) high(0, nx * plane + m, 1);
+            if (j == ny - 1) high(1, idx3(i, ny, k, ny + 1, nz), 3);
+            if (k == nz - 1) high(2, idx3(i, j, nz, ny, nz + 1), 5);
         }
     }
 }
@@ -2018,6 +2044,15 @@ inline int cu(cudaError_t e) { return e == cudaSuccess ? EDGE_OK : (int)e; }
 // blocks (8 per SM), which bounds the last-block atomics
 constexpr int kMaxBlocks = 148 * 8;
 inline int rgrid(long long n) { return (int)std::max<long long>(1, std::min<long long>(grid_for(n), kMaxBlocks)); }
+
+// Four cells of a line per thread where that leaves a wave of threads, two
+// below (a solve of 32^3: 388 us with two, 392 us with four).
+template <class F>
+void with_lines(const Lvl& L, F f) {
+    const long long n = (long long)L.n0 * L.n1 * L.n2;
+    if (n >= 1 << 20) f(std::integral_constant<int, 4>(), rgrid((long long)L.n1 * L.n2 * ((L.n0 + 3) / 4)));
+    else f(std::integral_constant<int, 2>(), rgrid((long long)L.n1 * L.n2 * ((L.n0 + 1) / 2)));
+}
 
 // plane length rounded to 64 floats, so every plane starts 256-byte aligned
 inline size_t plane_alloc(long long P) { return (size_t)((P + 63) / 64 * 64); }
@@ -2430,8 +2465,11 @@ void enqueue_setup(Solver* s, Faces U, const float* rhs, double abs_tol, double 
         }
     }
     cudaMemsetAsync(c.g.st->counter, 0, sizeof(c.g.st->counter), cs);  // fresh reduction counters
-    if (s->solid) k_setup_rhs<true><<<rgrid(L0.P), 256, 0, cs>>>(c.g, L0, c.f, U, rhs, abs_tol, rel_tol, max_iters);
-    else k_setup_rhs<false><<<rgrid(L0.P), 256, 0, cs>>>(c.g, L0, c.f, U, rhs, abs_tol, rel_tol, max_iters);
+    with_lines(L0, [&](auto line, int blocks) {
+        constexpr int N = decltype(line)::value;
+        if (s->solid) k_setup_rhs<true, N><<<blocks, 256, 0, cs>>>(c.g, L0, c.f, U, rhs, abs_tol, rel_tol, max_iters);
+        else k_setup_rhs<false, N><<<blocks, 256, 0, cs>>>(c.g, L0, c.f, U, rhs, abs_tol, rel_tol, max_iters);
+    });
     if (s->solid && !rhs) k_solid_fix<<<rgrid(L0.P), 256, 0, cs>>>(c.g, L0, c.f);
     if (stepwise) enqueue_step_pl(c, s->solid, cs, true);  // the stepwise solve: the first V-cycle's descent
     else enqueue_vcycle(c, s->solid, cs, true);          // first preconditioner application + z.r + tol
@@ -2444,7 +2482,9 @@ void enqueue_finish(Solver* s, Faces U, const float* rhs, float* xout, cudaStrea
     int n = L0.n0 * L0.n1 * L0.n2;
     int nx = s->nx, ny = s->ny, nz = s->nz;
     if (!rhs) {
-        k_grad_p<<<rgrid(L0.P), 256, 0, cs>>>(c.g, L0, c.f, U);
+        with_lines(L0, [&](auto line, int blocks) {
+            k_grad_p<decltype(line)::value><<<blocks, 256, 0, cs>>>(c.g, L0, c.f, U);
+        });
         if (s->solid) k_apply_solid<<<grid_for(n), 256, 0, cs>>>(c.g.st, nx, ny, nz, L0.bm, s->bvel, U);
     } else {
         k_from_rb<<<rgrid(n), 256, 0, cs>>>(c.g.st, L0, c.f.x[0], c.f.x[1], xout, &c.g.st->x_valid, 0, nullptr);
