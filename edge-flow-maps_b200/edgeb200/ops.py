@@ -82,6 +82,8 @@ def reset_faces(res, dx, phi, Fm):
 def march_edge(u, dx, dt, eps, psi, T, dT, opsi, oT, odT, identity=False, update=False):
     """update: psi, T and dT receive the results as well."""
     nx, ny, nz = cell_dims(opsi)
+    if update:
+        _check_update((opsi, *oT, *odT), (psi, *T, *dT))
     work = None if identity else _map_workspace(opsi)
     args = [nx, ny, nz, F(dx), F(dt), F(eps), *_p3(u), ptr(psi), *_p3(T), *_p3(dT), ptr(opsi), *_p3(oT), *_p3(odT)]
     if work is None:
@@ -96,6 +98,8 @@ def march_edge(u, dx, dt, eps, psi, T, dT, opsi, oT, odT, identity=False, update
 def march_ed4(u, dx, dt, eps, psi, T, opsi, oT, update=False):
     """update: psi and T receive the results as well."""
     nx, ny, nz = cell_dims(opsi)
+    if update:
+        _check_update((opsi, *oT), (psi, *T))
     work = _map_workspace(opsi)
     args = [nx, ny, nz, F(dx), F(dt), F(eps), *_p3(u), ptr(psi), *_p3(T)]
     if work is None:
@@ -106,6 +110,14 @@ def march_ed4(u, dx, dt, eps, psi, T, opsi, oT, update=False):
     else:
         _call("edge_march_fields", 0, *args, *_p3(None), ptr(opsi), *_p3(oT), *_p3(None), int(bool(update)), ptr(work),
               stream())
+
+
+def _check_update(new, old):
+    """The kernel writes the accumulated map by the new one's dimensions, so
+    both must have them (`copy` checks the same where it does the writing)."""
+    for s, d in zip(new, old):
+        if s.numel() != d.numel():
+            raise ValueError("march: the accumulated map and the new one must have one size (size mismatch)")
 
 
 def _map_workspace(psi):

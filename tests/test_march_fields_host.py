@@ -1,0 +1,26 @@
+"""What the marches of fields check and allocate on the host, before anything
+is launched (no GPU)."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+
+def _fields(res, count):
+    return [torch.zeros(res + (3,)) for _ in range(count)]
+
+
+# the results are written into the accumulated map by the dimensions of the new
+# one: a map of another size has to be refused, as a copy refuses it
+@pytest.mark.parametrize("at", range(7))
+@pytest.mark.parametrize("other", [(8, 8, 6), (8, 8, 12)])
+def test_accumulated_map_of_another_size_is_refused(at, other):
+    from sim import hermite
+    res, dx = (8, 8, 8), 0.125
+    u = [torch.zeros(s) for s in ((9, 8, 8), (8, 9, 8), (8, 8, 9))]
+    acc = _fields(res, 7)
+    acc[at] = _fields(other, 1)[0]
+    with pytest.raises(ValueError, match="size mismatch"):
+        hermite.advect_psi_garm_ed4_fusion_unroll(*_fields(res, 7), *acc, *u, None, dx, 0.01, 0.01)
+    if at < 4:
+        with pytest.raises(ValueError, match="size mismatch"):
+            hermite.advect_ps_hermite_ed4_fd_unroll(*_fields(res, 4), *acc[:4], *u, None, dx, 0.01, 0.01)
