@@ -128,7 +128,7 @@ def _map_workspace(psi):
     100x75x61 543 and 405, 256x128x128 4850 and 2847; ED4 38 and 34, 88 and 50,
     541 and 239, 4122 and 1734)."""
     try:
-        return torch.empty((8, psi.numel() // 3, 4), device=psi.device)
+        return torch.empty((8, psi.numel() // 3, 4), dtype=torch.float32, device=psi.device)
     except torch.cuda.OutOfMemoryError:
         return None
 

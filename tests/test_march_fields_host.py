@@ -24,3 +24,17 @@ def test_accumulated_map_of_another_size_is_refused(at, other):
     if at < 4:
         with pytest.raises(ValueError, match="size mismatch"):
             hermite.advect_ps_hermite_ed4_fd_unroll(*_fields(res, 4), *acc[:4], *u, None, dx, 0.01, 0.01)
+
+
+# the packed copy of the map is float32 whatever torch's default type is
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float16, torch.bfloat16, torch.float32])
+def test_scratch_under_another_default_dtype(dtype):
+    from edgeb200 import ops
+    before = torch.get_default_dtype()
+    psi = torch.zeros((4, 5, 6, 3), dtype=torch.float32)
+    torch.set_default_dtype(dtype)
+    try:
+        work = ops._map_workspace(psi)
+    finally:
+        torch.set_default_dtype(before)
+    assert work.dtype == torch.float32 and work.numel() == 8 * 4 * 4 * 5 * 6
