@@ -39,7 +39,7 @@ __global__ void k_points_mac(Mac mac, const float* __restrict__ pts, int n, floa
     if (e >= n) return;
     float p[3] = {pts[3 * e], pts[3 * e + 1], pts[3 * e + 2]};
     float a[3], b[3], G[3][3];
-    mac_sample_points(mac, p, a);
+    mac_sample_points(mac, p, lanes_below(e, n), a);
     mac_sample<true>(mac, p, b, G);
     for (int c = 0; c < 3; c++) {
         v[3 * e + c] = a[c];

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../../include/edge_b200.h"
 
 #define EDGE_HD __host__ __device__ __forceinline__
@@ -176,23 +178,22 @@ EDGE_D GRows grows(const float* f, int x, int y, int z, int n1, int n2) {
     return GRows{f, idx3(x, y, z, n1, n2), n1, n2};
 }
 
-// The taps of samples at scattered points.  A warp's load there costs a
-// wavefront for every point or two, whatever its width, and 81 of them per
-// point were the bound: a row's three taps come in the aligned 16 bytes that
-// hold the first and, where these do not hold the third, the 8 bytes after
-// them.  `wide`: no such load passes either end of the field.  200 000 points
-// at random in 256x128x128 39 -> 32.5 us.
+// The taps of samples at scattered points, which take 64-bit addresses.  Where
+// a warp's points are in no order, its load costs a wavefront for every point
+// or two, whatever its width: WIDE takes a row's three taps in the aligned 16
+// bytes that hold the first and, where these do not hold the third, the 8 bytes
+// after them.
 struct VRow {
     float q[3];
     EDGE_D float operator[](int k) const { return q[k]; }
 };
+template <bool WIDE>
 struct VRows {
     const float* f;  // the sample's first tap
     int n1, n2;
-    bool wide;
     EDGE_D VRow operator()(int i, int j) const {
         const float* p = f + (i * n1 + j) * n2;
-        if (!wide) return VRow{{__ldg(p), __ldg(p + 1), __ldg(p + 2)}};
+        if (!WIDE) return VRow{{__ldg(p), __ldg(p + 1), __ldg(p + 2)}};
         const unsigned o = (unsigned)(reinterpret_cast<size_t>(p) >> 2) & 3;
         const float4 a = __ldg(reinterpret_cast<const float4*>(p - o));
         float2 b = make_float2(0.f, 0.f);
@@ -202,9 +203,12 @@ struct VRows {
         return (o & 2) ? VRow{{s2, s3, s4}} : VRow{{s0, s1, s2}};
     }
 };
-EDGE_D VRows vrows(const float* f, int x, int y, int z, int n0, int n1, int n2) {
-    const long long e = ((long long)x * n1 + y) * n2 + z, last = e + (2LL * n1 + 2) * n2 + 2;
-    return VRows{f + e, n1, n2, e >= 3 && last + 3 < (long long)n0 * n1 * n2};
+// whether the rows of a sample whose first tap is (x, y, .) have another row of
+// the field before and after them, so that no wide load passes its ends
+EDGE_D bool rows_inside(int x, int y, int n0, int n1) { return (x > 0 || y > 0) && (x + 3 < n0 || y + 3 < n1); }
+template <bool WIDE>
+EDGE_D VRows<WIDE> vrows(const float* f, int x, int y, int z, int n1, int n2) {
+    return VRows<WIDE>{f + (((long long)x * n1 + y) * n2 + z), n1, n2};
 }
 
 // 27-tap separable contraction of one scalar field, z then y then x, value and
@@ -273,6 +277,24 @@ EDGE_D float bspline_sum(const Rows& rows, const Axis3<false>& X, const Axis3<fa
     return __fmaf_rn(X.w[2], c2, v);
 }
 
+// The same value row by row: fewer registers, for the samplers at scattered
+// points, where more warps in flight are worth more than a warp's loads ahead.
+template <class Rows>
+EDGE_D float bspline_rows(const Rows& rows, const Axis3<false>& X, const Axis3<false>& Y, const Axis3<false>& Z) {
+    float v = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        float c = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const auto q = rows(i, j);
+            c = __fmaf_rn(Y.w[j], dot3(Z.w[0], q[0], Z.w[1], q[1], Z.w[2], q[2]), c);
+        }
+        v = __fmaf_rn(X.w[i], c, v);
+    }
+    return v;
+}
+
 // MAC velocity field + the clamp bounds of its three staggered components.
 struct Mac {
     const float* __restrict__ u[3];
@@ -317,17 +339,39 @@ EDGE_D void mac_sums(const Mac& m, const Axis3<GRAD> A0[3], const Axis3<GRAD> A5
                        m.inv_dx, GRAD ? G[2] : nullptr);
 }
 
-// interp_u_MAC at a scattered point.
-EDGE_D void mac_sample_points(const Mac& m, const float p[3], float v[3]) {
+// interp_u_MAC at a scattered point; mask: the warp's lanes that sample.  A
+// warp's points in no order are bound by wavefronts and take wide loads; points
+// that follow one another in space (sorted particles, a lattice) share their
+// lines, and there a 16-byte load, which goes by quarters of a warp, costs more
+// wavefronts than three scalar ones.  So a warp takes wide loads where more than
+// kPointGroups of its points lie apart from the one before.  us, always wide,
+// always scalar and so: 10^6 points at random in 128x256x128 135, 164, 131; in
+// a ball 115, 148, 113; on a lattice 88, 31, 37; sorted by cell 85, 48, 51; in
+// runs of two 89, 87, 78, of four 90, 52, 55.
+constexpr int kPointGroups = 10;
+EDGE_D void mac_sample_points(const Mac& m, const float p[3], unsigned mask, float v[3]) {
     float q[3];
     Axis3<false> A0[3], A5[3];
     mac_axes<false>(m, p, q, A0, A5);
-    v[0] = bspline_sum(vrows(m.u[0], A0[0].base, A5[1].base, A5[2].base, m.nx + 1, m.ny, m.nz), A0[0], A5[1], A5[2],
-                       m.inv_dx, nullptr);
-    v[1] = bspline_sum(vrows(m.u[1], A5[0].base, A0[1].base, A5[2].base, m.nx, m.ny + 1, m.nz), A5[0], A0[1], A5[2],
-                       m.inv_dx, nullptr);
-    v[2] = bspline_sum(vrows(m.u[2], A5[0].base, A5[1].base, A0[2].base, m.nx, m.ny, m.nz + 1), A5[0], A5[1], A0[2],
-                       m.inv_dx, nullptr);
+    const int x0 = A0[0].base, y0 = A0[1].base, z0 = A0[2].base, x5 = A5[0].base, y5 = A5[1].base, z5 = A5[2].base;
+    const int xy = (x0 << 16) ^ y0, bxy = __shfl_up_sync(mask, xy, 1), bz = __shfl_up_sync(mask, z0, 1);
+    const bool apart = abs((xy >> 16) - (bxy >> 16)) > 1 || abs((xy & 0xffff) - (bxy & 0xffff)) > 1 || abs(z0 - bz) > 16;
+    const bool inside = rows_inside(x0, y5, m.nx + 1, m.ny) && rows_inside(x5, y0, m.nx, m.ny + 1) &&
+                        rows_inside(x5, y5, m.nx, m.ny);
+    auto sums = [&](auto wide) {
+        constexpr bool W = decltype(wide)::value;
+        v[0] = bspline_rows(vrows<W>(m.u[0], x0, y5, z5, m.ny, m.nz), A0[0], A5[1], A5[2]);
+        v[1] = bspline_rows(vrows<W>(m.u[1], x5, y0, z5, m.ny + 1, m.nz), A5[0], A0[1], A5[2]);
+        v[2] = bspline_rows(vrows<W>(m.u[2], x5, y5, z0, m.ny, m.nz + 1), A5[0], A5[1], A0[2]);
+    };
+    if (__popc(__ballot_sync(mask, apart)) > kPointGroups && __all_sync(mask, inside)) sums(std::true_type{});
+    else sums(std::false_type{});
+}
+// the lanes of a warp (of a one-dimensional block) whose index is below n, for
+// a thread e that is one of them
+EDGE_D unsigned lanes_below(int e, int n) {
+    const int left = n - (e - (int)(threadIdx.x & 31));
+    return left >= 32 ? 0xffffffffu : (1u << left) - 1u;
 }
 
 // interp_u_MAC / interp_u_MAC_grad (taichi_utils.py:322-341).  G rows are the
