@@ -76,11 +76,9 @@ __global__ void __launch_bounds__(kPointBlock, 9) k_lp_vel_diff(Mac mac_, const 
 // B-spline scatter of the drag onto the three face grids (atomic adds, like
 // the reference's `+=` in a parallel loop)
 template <bool P2>
-__global__ void k_lp_p2g(int nx, int ny, int nz, float dx, float inv_dx, float* dx_, float* dy_, float* dz_,
-                         const float* __restrict__ vdiff, const float* __restrict__ pos,
-                         const float* __restrict__ rad, int num, float lrad, float Lx, float Ly, float Lz) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= num) return;
+EDGE_D void scatter_particle(int e, int nx, int ny, int nz, float dx, float inv_dx, float* dx_, float* dy_, float* dz_,
+                             const float* __restrict__ vdiff, const float* __restrict__ pos,
+                             const float* __restrict__ rad, float lrad, float Lx, float Ly, float Lz) {
     float p[3] = {pos[3 * e], pos[3 * e + 1], pos[3 * e + 2]};
     if (p[0] < 3 * dx || p[1] < 3 * dx || p[2] < 3 * dx || p[0] > Lx - 3 * dx || p[1] > Ly - 3 * dx ||
         p[2] > Lz - 3 * dx)
@@ -129,6 +127,14 @@ __global__ void k_lp_p2g(int nx, int ny, int nz, float dx, float inv_dx, float* 
         }
     }
 }
+template <bool P2>
+__global__ void k_lp_p2g(int nx, int ny, int nz, float dx, float inv_dx, float* dx_, float* dy_, float* dz_,
+                         const float* __restrict__ vdiff, const float* __restrict__ pos,
+                         const float* __restrict__ rad, int num, float lrad, float Lx, float Ly, float Lz) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < num)
+        scatter_particle<P2>(e, nx, ny, nz, dx, inv_dx, dx_, dy_, dz_, vdiff, pos, rad, lrad, Lx, Ly, Lz);
+}
 
 // ---------------------------------------------------------------------------
 // The same scatter through particles grouped by cell.  k_lp_p2g adds every
@@ -155,7 +161,7 @@ struct P2G {
     int* key;    // cell of a particle, -1 where it does not scatter
     int* rank;   // its place among the cell's particles
     int* order;  // the particles, grouped by cell
-    int* total;  // [0] particles grouped, [1] cells that hold any
+    int* total;  // [0] particles grouped, [1] whether they scatter directly instead
 };
 
 template <bool P2>
@@ -170,10 +176,60 @@ EDGE_D bool p2g_coord(const P2G& a, int e, float g[3]) {
     return in;
 }
 
+// Zeroes the drag and the counts, and looks whether grouping pays.  The direct
+// scatter is bound by the sectors that a warp's atomics fall on and by particles
+// that share a face.  In an order where they follow one another cell by cell (a
+// lattice, a line) both are few and it is the faster one; so it is where none
+// reaches a face.  16 warps of consecutive particles are looked at: their cells,
+// and the sectors of their first staggered taps, which alternate between rows
+// where the particles lie at random in sorted cells.  us, direct, grouped and
+// so: 10^6 on a lattice in 192x96x96 138, 281, 142, in 128x256x128 178, 302, 188;
+// 200 000 in 64^3 35, 69, 40; sorted by cell in 192x96x96 348, 233, 232; at
+// random 541, 247, 245; 10^6 out of reach 12, 23, 18.
 template <bool P2>
-__global__ void __launch_bounds__(256) k_p2g_count(P2G a) {
+__global__ void __launch_bounds__(512) k_p2g_begin(P2G a, float* Dx, float* Dy, float* Dz) {
+    if (blockIdx.x == 0) {
+        const unsigned lane = threadIdx.x & 31, before = (1u << lane) - 1u;
+        // multiples of the golden ratio: no lattice's period
+        const unsigned at = (threadIdx.x >> 5) * 0x9e3779b9u;
+        const int e = (int)((unsigned long long)at * (unsigned)max(a.num - 31, 1) >> 32) + (int)lane;
+        float g[3];
+        const bool in = e < a.num && p2g_coord<P2>(a, e, g);
+        const unsigned mask = __ballot_sync(0xffffffffu, in);
+        bool direct = false;
+        if (in) {
+            const int cell = idx3((int)g[0], (int)g[1], (int)g[2], a.ny, a.nz),
+                      face = idx3((int)(g[0] - 0.5f), (int)(g[1] - 0.5f), (int)(g[2] - 0.5f), a.ny, a.nz);
+            const int all = __popc(mask), cells = __popc(__ballot_sync(mask, !(__match_any_sync(mask, cell) & before))),
+                      sectors = __popc(__ballot_sync(mask, !(__match_any_sync(mask, face >> 3) & before)));
+            direct = 8 * cells >= 5 * all && 8 * sectors <= 3 * all + 8;
+        }
+        const int reach = __syncthreads_count(in), yes = __syncthreads_count(direct);
+        if (threadIdx.x == 0) {
+            a.total[0] = 0;
+            a.total[1] = 2 * yes >= reach;
+        }
+    }
+    const int n = a.nx * a.ny * a.nz;
+    const long long fx = n + (long long)a.ny * a.nz, fy = n + (long long)a.nx * a.nz, fz = n + (long long)a.nx * a.ny,
+                    step = (long long)gridDim.x * blockDim.x;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < fx || t < fy || t < fz; t += step) {
+        if (t < fx) Dx[t] = 0.0f;
+        if (t < fy) Dy[t] = 0.0f;
+        if (t < fz) Dz[t] = 0.0f;
+        if (t < n) a.cell[t] = 0;
+    }
+}
+
+template <bool P2>
+__global__ void __launch_bounds__(256) k_p2g_count(P2G a, float* Dx, float* Dy, float* Dz) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= a.num) return;
+    if (a.total[1]) {
+        scatter_particle<P2>(e, a.nx, a.ny, a.nz, a.dx, a.inv_dx, Dx, Dy, Dz, a.vdiff, a.pos, a.rad, a.lrad, a.L[0],
+                             a.L[1], a.L[2]);
+        return;
+    }
     float g[3];
     int key = -1;
     if (p2g_coord<P2>(a, e, g)) {
@@ -188,38 +244,32 @@ __global__ void __launch_bounds__(256) k_p2g_count(P2G a) {
 
 // counts to segment starts; one atomic on the running total per block
 __global__ void __launch_bounds__(256) k_p2g_start(int n, int* cell, int* total) {
-    __shared__ int warp_sum[8], warp_occ[8], base;
+    if (total[1]) return;
+    __shared__ int warp_sum[8], base;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int e0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    int c[4], s = 0, occ = 0;
+    int c[4], s = 0;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         c[q] = e0 + q < n ? cell[e0 + q] : 0;
         s += c[q];
-        occ += c[q] > 0;
     }
     int incl = s;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int t = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += t;
-        occ += __shfl_xor_sync(0xffffffffu, occ, o);
     }
-    if (lane == 31) {
-        warp_sum[w] = incl;
-        warp_occ[w] = occ;
-    }
+    if (lane == 31) warp_sum[w] = incl;
     __syncthreads();
     if (threadIdx.x == 0) {
-        int t = 0, u = 0;
+        int t = 0;
         for (int q = 0; q < 8; q++) {
             const int v = warp_sum[q];
             warp_sum[q] = t;
             t += v;
-            u += warp_occ[q];
         }
         base = t ? atomicAdd(total, t) : 0;
-        if (u) atomicAdd(total + 1, u);
     }
     __syncthreads();
     int at = base + warp_sum[w] + incl - s;
@@ -230,12 +280,11 @@ __global__ void __launch_bounds__(256) k_p2g_start(int n, int* cell, int* total)
     }
 }
 
-__global__ void __launch_bounds__(256) k_p2g_place(int num, const int* __restrict__ cell, const int* __restrict__ key,
-                                                   const int* __restrict__ rank, int* order) {
+__global__ void __launch_bounds__(256) k_p2g_place(P2G a) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= num) return;
-    const int k = key[e];
-    if (k >= 0) order[cell[k] + rank[e]] = e;
+    if (e >= a.num || a.total[1]) return;
+    const int k = a.key[e];
+    if (k >= 0) a.order[a.cell[k] + a.rank[e]] = e;
 }
 
 constexpr int kSumWarps = 4;
@@ -447,11 +496,8 @@ int edge_lp_p2g_grouped(int nx, int ny, int nz, float dx, float* dragx, float* d
     if (!dragx || !dragy || !dragz || (num && (!vdiff || !pos || !rad)) || !work || work_bytes < need) return EDGE_EINVAL;
     if ((uintptr_t)work & 15) return EDGE_EALIGN;
     cudaStream_t s = S(stream);
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(dragx, 0, (size_t)(nx + 1) * ny * nz * 4, s)) != cudaSuccess) return (int)e;
-    if ((e = cudaMemsetAsync(dragy, 0, (size_t)nx * (ny + 1) * nz * 4, s)) != cudaSuccess) return (int)e;
-    if ((e = cudaMemsetAsync(dragz, 0, (size_t)nx * ny * (nz + 1) * 4, s)) != cudaSuccess) return (int)e;
-    if (num == 0) return EDGE_OK;
+    if (num == 0)
+        return edge_lp_p2g(nx, ny, nz, dx, dragx, dragy, dragz, vdiff, pos, rad, 0, laden_radius, Lx, Ly, Lz, stream);
     const int n = nx * ny * nz;
     char* w = (char*)work;
     P2G a;
@@ -467,15 +513,17 @@ int edge_lp_p2g_grouped(int nx, int ny, int nz, float dx, float* dragx, float* d
     a.rank = (int*)w;
     w += p2g_part(num);
     a.order = (int*)w;
-    if ((e = cudaMemsetAsync(a.cell, 0, ((size_t)n + 2) * 4, s)) != cudaSuccess) return (int)e;
     // a warp walks over more than one batch when that still leaves 32 warps per SM
     const int batches = (int)std::max(1LL, std::min(8LL, num / (32LL * 32 * 148)));
     const int warps = grid_for(num, 32 * batches);
     const bool p2 = pow2f(dx);
-    if (p2) k_p2g_count<true><<<grid_for(num), 256, 0, s>>>(a);
-    else k_p2g_count<false><<<grid_for(num), 256, 0, s>>>(a);
+    const int zero = std::min(grid_for(n, 1024), 148 * 4);
+    if (p2) k_p2g_begin<true><<<zero, 512, 0, s>>>(a, dragx, dragy, dragz);
+    else k_p2g_begin<false><<<zero, 512, 0, s>>>(a, dragx, dragy, dragz);
+    if (p2) k_p2g_count<true><<<grid_for(num), 256, 0, s>>>(a, dragx, dragy, dragz);
+    else k_p2g_count<false><<<grid_for(num), 256, 0, s>>>(a, dragx, dragy, dragz);
     k_p2g_start<<<grid_for(n, 1024), 256, 0, s>>>(n, a.cell, a.total);
-    k_p2g_place<<<grid_for(num), 256, 0, s>>>(num, a.cell, a.key, a.rank, a.order);
+    k_p2g_place<<<grid_for(num), 256, 0, s>>>(a);
     if (p2) k_p2g_sum<true><<<grid_for(warps, kSumWarps), 32 * kSumWarps, 0, s>>>(a, dragx, dragy, dragz, batches);
     else k_p2g_sum<false><<<grid_for(warps, kSumWarps), 32 * kSumWarps, 0, s>>>(a, dragx, dragy, dragz, batches);
     return st();

@@ -18,7 +18,7 @@ F = ctypes.c_float
 
 # kernels each entry point launches (memcpy/memset nodes are not counted)
 _KERNELS = {"edge_max_speed": 2, "edge_copy": 0, "edge_lp_max_speed": 2, "edge_march_ge": 3,
-            "edge_march_ge_packed": 3, "edge_calc_fd_3_from_grad": 2, "edge_lp_p2g_grouped": 4, "edge_march_fields": 3}
+            "edge_march_ge_packed": 3, "edge_calc_fd_3_from_grad": 2, "edge_lp_p2g_grouped": 5, "edge_march_fields": 3}
 _launched = [0]
 
 
@@ -316,9 +316,9 @@ def lp_vel_diff(u, dx, vel, vdiff, pos, num, St, density_ratio, epiral_radius_ra
 def lp_p2g(res, dx, drag, vdiff, pos, rad, num, laden_radius, L):
     num, n = int(num), int(res[0]) * int(res[1]) * int(res[2])
     tail = [ptr(vdiff), ptr(pos), ptr(rad), num, F(laden_radius), *[F(v) for v in L]]
-    # the grouped scatter costs some 20 us of launches and a pass over the cells more; measured (us, direct / grouped):
-    # 20000 particles 45 / 60 (4.2 M cells), 42 / 42 (64^3); 50000 75 / 42 (10^5 cells); 100000 105 / 70, 262144 224 / 121
-    # and 10^6 642 / 302 (4.2 M cells, 1 to 2 per cell); 10^6 at 18 per cell 746 / 140
+    # the grouped scatter costs four launches and a pass over the cells more; device time (us, direct / grouped):
+    # in a ball, 40000 particles 55 / 25 (262144 cells), 50000 58 / 31 (1.8 M), 70000 70 / 49 (4.2 M); at random,
+    # 40000 36 / 31, 200000 133 / 70, 10^6 562 / 294
     work = _p2g_workspace(res, num, pos.device) if num >= 32768 + n // 128 and n < 2 ** 31 else None
     if work is None:
         _call("edge_lp_p2g", *res, F(dx), *_p3(drag), *tail, stream())

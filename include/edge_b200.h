@@ -442,8 +442,10 @@ int edge_lp_p2g(int nx, int ny, int nz, float dx, float *dragx, float *dragy, fl
                 const float *pos, const float *rad, int num, float laden_radius, float Lx, float Ly, float Lz,
                 void *stream);
 /* The same scatter with the particles grouped by cell first, their sums per
- * cell formed before the atomic adds: the faster one where several particles
- * share a cell.  work: device memory of at least the size that
+ * cell formed before the atomic adds: the faster one for particles in no order
+ * and where several share a cell.  Where the particles follow one another cell
+ * by cell, as on a lattice, the call scatters directly after all; it looks at
+ * some of them on the device.  work: device memory of at least the size that
  * edge_lp_p2g_workspace gives, 16-byte aligned, free again when the call's
  * work on the stream is done. */
 int edge_lp_p2g_workspace(int nx, int ny, int nz, int num, long long *bytes);
