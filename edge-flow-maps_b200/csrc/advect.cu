@@ -402,10 +402,17 @@ __global__ void __launch_bounds__(128) k_march_ed8_p(Mac mac_, MapP m_, float dt
 // (hermite.py:643-654, 864-918 with -dt) and composed with the accumulated
 // map through the full stored-derivative Hermite (hermite.py:1024-1046).
 // dT and d2T of the new map come from calc_fd_3_from_grad afterwards.
-EDGE_D void herm_full(const MapF& m, const float p[3], float v[3], float g[3][3]) { hermite3<HV_FULL, true>(m, p, v, g); }
-EDGE_D void herm_full(const MapP& m, const float p[3], float v[3], float g[3][3]) { hermite3p_pairs<HV_FULL>(m, p, v, g); }
+template <bool PAIRS>
+EDGE_D void herm_full(const MapF& m, const float p[3], float v[3], float g[3][3]) {
+    hermite3<HV_FULL, true>(m, p, v, g);
+}
+template <bool PAIRS>
+EDGE_D void herm_full(const MapP& m, const float p[3], float v[3], float g[3][3]) {
+    if (PAIRS) hermite3p_pairs<HV_FULL>(m, p, v, g);
+    else hermite3p<HV_FULL, true>(m, p, v, g);
+}
 
-template <bool F64 = false, class M>
+template <bool PAIRS, class M>
 EDGE_D void ge_center(const Mac& mac, const M& m, int i, int j, int k, float dt, float P[3], float (&T)[3][3]) {
     cell_pos(i, j, k, m.dx, P);
     float C[3][3];
@@ -413,8 +420,8 @@ EDGE_D void ge_center(const Mac& mac, const M& m, int i, int j, int k, float dt,
         for (int d = 0; d < 3; d++) C[c][d] = c == d ? 1.0f : 0.0f;
     rk4_jac<3>(mac, P, C, -dt);
     float val[3], G[3][3];
-    herm_full(m, P, val, G);
-    compose_jac<F64>(G, C, T);  // T = T_old @ T_step
+    herm_full<PAIRS>(m, P, val, G);
+    compose_jac<false>(G, C, T);  // T = T_old @ T_step
     for (int c = 0; c < 3; c++) P[c] = val[c];
 }
 
@@ -424,7 +431,7 @@ __global__ void __launch_bounds__(128) k_march_ge(Mac mac, MapF m, float dt, flo
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= m.nx * m.ny * m.nz) return;
     float P[3], T[3][3];
-    ge_center(mac, m, e / (m.ny * m.nz), (e / m.nz) % m.ny, e % m.nz, dt, P, T);
+    ge_center<false>(mac, m, e / (m.ny * m.nz), (e / m.nz) % m.ny, e % m.nz, dt, P, T);
     float* oT[3] = {oTx, oTy, oTz};
     for (int c = 0; c < 3; c++) {
         opsi[3 * e + c] = P[c];
@@ -432,18 +439,23 @@ __global__ void __launch_bounds__(128) k_march_ge(Mac mac, MapF m, float dt, flo
     }
 }
 
-// packed layout: planes 0-3 of `out`.  Four samples per cell are too few to
-// pay for a tile; paired contractions at five blocks per SM: 256x128x128 747 ->
-// 715 us, 192x96x96 352 -> 321 us.
-template <bool P2>
-__global__ void __launch_bounds__(128, 5) k_march_ge_p(Mac mac_, MapP m_, float dt, float4* __restrict__ out) {
+// packed layout: planes 0-3 of `out`.  Four samples per cell are too few to pay
+// for a tile.  Registers or warps decide (us: scalar uncapped, pairs uncapped,
+// pairs at five blocks per SM, scalar at five): a grid of a wave or so wants the
+// registers (64x32x32 21.2, 20.8, 22.6, 22.2; 48^3 28.7, 26.8, 29.5, 32.8; 60^3
+// pairs 47 and 49), above that pairs at five blocks where the spacing is no power
+// of two (96^3 205, 170, 164, 180) and scalar ones where it is (64^3 57.4, 57.4,
+// 55.5, 53.5; 256x128x128 807, 838, 712, 702).  Positions, spacings and the
+// contraction's order are the same, and so are the bits.
+template <bool PAIRS, int BLOCKS, bool P2>
+__global__ void __launch_bounds__(128, BLOCKS) k_march_ge_p(Mac mac_, MapP m_, float dt, float4* __restrict__ out) {
     const Mac mac = with_pow2<P2>(mac_);
     const MapP m = with_pow2<P2>(m_);
     int e = blockIdx.x * blockDim.x + threadIdx.x;
     const int n = m.n;
     if (e >= n) return;
     float P[3], T[3][3];
-    ge_center(mac, m, e / (m.ny * m.nz), (e / m.nz) % m.ny, e % m.nz, dt, P, T);
+    ge_center<PAIRS>(mac, m, e / (m.ny * m.nz), (e / m.nz) % m.ny, e % m.nz, dt, P, T);
     out[e] = make_float4(P[0], P[1], P[2], 0.f);
 #pragma unroll
     for (int d = 0; d < 3; d++) out[(size_t)(1 + d) * n + e] = make_float4(T[0][d], T[1][d], T[2][d], 0.f);
@@ -1488,8 +1500,9 @@ int edge_march_ge_packed(int nx, int ny, int nz, float dx, float dt, const float
     const int n = nx * ny * nz;
     float4* o = (float4*)out_packed;
     const Mac mac = make_mac(ux, uy, uz, nx, ny, nz, dx);
-    if (mac.pow2) k_march_ge_p<true><<<grid_for(n, 128), 128, 0, S(stream)>>>(mac, m, dt, o);
-    else k_march_ge_p<false><<<grid_for(n, 128), 128, 0, S(stream)>>>(mac, m, dt, o);
+    auto launch = [&](auto k) { k<<<grid_for(n, 128), 128, 0, S(stream)>>>(mac, m, dt, o); };
+    if (n <= (mac.pow2 ? 98304 : 262144)) launch(mac.pow2 ? k_march_ge_p<true, 1, true> : k_march_ge_p<true, 1, false>);
+    else launch(mac.pow2 ? k_march_ge_p<false, 5, true> : k_march_ge_p<true, 5, false>);
     k_fd3_dT_p<<<grid_for(n), kBlock, 0, S(stream)>>>(nx, ny, nz, dx, o);
     k_fd3_d2T_p<<<grid_for(n), kBlock, 0, S(stream)>>>(nx, ny, nz, dx, o);
     return launch_status();
