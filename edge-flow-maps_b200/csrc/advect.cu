@@ -1699,10 +1699,16 @@ int edge_advect_u_sl(int nx, int ny, int nz, float dx, float dt, const float* ux
     const int tiles = tile_blocks<CellTile>(nx, ny, nz);
     // by tiles a thread takes three faces in turn, which needs enough tiles to
     // fill the device, and tiles that the grid fills (us, consecutive faces and
-    // tiles: 64^3 51 and 60, 97x65x49 70 and 70, 100x75x61 96 and 88,
-    // 192x96x96 340 and 322, 256x128x128 752 and 663)
+    // tiles: 64^3 51 and 60, 97x65x49 70 and 70, 100x75x61 97 and 88,
+    // 192x96x96 339 and 317, 256x128x128 746 and 651).  Rows of whole 128-byte
+    // lines put a warp's taps on fewer wavefronts, and consecutive faces keep up
+    // longer (80x72x64 70 and 76, 128x64x64 96 and 99, 160x64x64 119 and 119,
+    // 96^3 172 and 165).  Samples that leave their tile cost more than without
+    // one there, which is a matter of steps of two cells and more: 128x128x64
+    // at two cells 193 and 194, at four 227 and 248; 256x128x128 at four 906 and
+    // 864, at eight 1172 and 1355; 100x75x61 at eight 178 and 158.
     const long long n = (long long)nx * ny * nz;
-    if (n >= 350000 && (double)n >= 0.8 * CellTile::threads * tiles) {
+    if (n >= (nz % 32 ? 350000 : 700000) && (double)n >= 0.8 * CellTile::threads * tiles) {
         const int g = tiles + grid_for((long long)ny * nz + (long long)nx * nz + (long long)nx * ny, CellTile::threads);
         if (mac.pow2) k_advect_tile<true, CellTile><<<g, CellTile::threads, 0, S(stream)>>>(mac, dt, ux1, uy1, uz1, tiles);
         else k_advect_tile<false, CellTile><<<g, CellTile::threads, 0, S(stream)>>>(mac, dt, ux1, uy1, uz1, tiles);
