@@ -1293,7 +1293,11 @@ inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 // fill at least `fill` of its threads: 0.9 for the EDGE march (us, NoTile and
 // tile: 96^3 715 and 657, 72x72x36 (0.90) 167 and 167, 97x65x49 (0.81) 279 and
 // 296), 0.8 for ED4 and ED8, whose samples weigh more (97x65x49 180 and 177,
-// 330 and 325; 80x48x40 92 and 91, 177 and 149).
+// 330 and 325; 80x48x40 92 and 91, 177 and 149).  A warp with a sample outside
+// its tile reads global memory, from four rows of eight cells instead of one of
+// 32, so steps of four cells and more, which no driver takes, cost more than
+// without tiles where rows are whole lines: 64x32x32 at four cells EDGE 80 and
+// 73, ED8 111 and 98, 64^3 EDGE 203 and 205, ED8 267 and 259.
 using CellTile = Tile<4, 4, 8>;
 template <class F>
 void with_tile(int nx, int ny, int nz, double fill, F f) {
@@ -1322,7 +1326,14 @@ void march_edge_by(const Mac& mac, const MapP& m, float dt, float eps, bool iden
 }
 template <class Out>
 void march_ed4_by(const Mac& mac, const MapP& m, float dt, float eps, Out out, cudaStream_t st) {
-    with_tile(mac.nx, mac.ny, mac.nz, 0.8, [&](auto t, int g) {
+    // Rows of whole 128-byte lines put a warp's global taps on few wavefronts,
+    // and with a spacing that needs no divisions the tile's staging is not
+    // earned back by sixteen samples up to half a million cells (us, tile and
+    // not: 32^3 35 and 31, 64x64x32 70 and 66, 64^3 120 and 117, 128x64x64 225
+    // and 225, 128x128x64 430 and 433; at four cells per step 32^3 43 and 35,
+    // 128x64x64 295 and 279).
+    const bool lines = mac.pow2 && mac.nz % 32 == 0 && m.n <= 1 << 19;
+    with_tile(mac.nx, mac.ny, mac.nz, lines ? 2.0 : 0.8, [&](auto t, int g) {
         using T = decltype(t);
         if (mac.pow2) k_march_ed4_p<true, T, Out><<<g, 128, 0, st>>>(mac, m, dt, eps, out);
         else k_march_ed4_p<false, T, Out><<<g, 128, 0, st>>>(mac, m, dt, eps, out);

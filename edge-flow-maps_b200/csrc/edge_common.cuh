@@ -409,8 +409,8 @@ EDGE_D float mac_sample_comp(const Mac& m, const float p[3], int a) {
 // nodes floor(q - 0.5) .. + 2 and, staggered, floor(q - 1) .. + 2, and the
 // clamped ones near the walls (a cell index is at most n - 1).  A warp with a
 // sample outside that takes it from global memory.  A step of up to a cell, as
-// the CFL condition gives, stays inside; at four cells, which no driver takes,
-// the marches of 64x32x32 cost up to a tenth more than without a tile.
+// the CFL condition gives, stays inside; what larger ones cost stands at the
+// rules that choose the tile.
 // ---------------------------------------------------------------------------
 // Blocks of 4 x 4 x 8 cells: 2 x 2 x 32 stage more nodes per cell, were slower
 // and leave more of a ragged grid's threads idle.
