@@ -628,6 +628,7 @@ __global__ void k_coef_p(MapP m, float4* __restrict__ g) {
 // 256x128x128: 818 us for one 64-coefficient launch per axis, 111 us so (the
 // copy bandwidth allows 90); 192x96x96, where a quarter of the faces is left
 // over: 363 and 218 us.
+
 // Hermite coordinate of axis d's cell centre i as hermite3p forms it: its base
 // cell, and whether it has no fractional part
 struct Centre {
@@ -1313,15 +1314,15 @@ void march_edge_by(const Mac& mac, const MapP& m, float dt, float eps, bool iden
     with_tile(mac.nx, mac.ny, mac.nz, 0.9, [&](auto t, int g) {
         using T = decltype(t);
         auto launch = [&](auto k) { k<<<g, 128, 0, st>>>(mac, m, dt, eps, out); };
-        if (mac.pow2) {
-            if (identity) launch(k_march_edge_p<true, false, true, T, Out>);
-            else if (f64) launch(k_march_edge_p<false, true, true, T, Out>);
-            else launch(k_march_edge_p<false, false, true, T, Out>);
-        } else {
-            if (identity) launch(k_march_edge_p<true, false, false, T, Out>);
-            else if (f64) launch(k_march_edge_p<false, true, false, T, Out>);
-            else launch(k_march_edge_p<false, false, false, T, Out>);
+        // the float64 composition exists on packed maps only
+        if constexpr (std::is_same_v<Out, PlanesOut>) {
+            if (f64 && !identity) {
+                launch(mac.pow2 ? k_march_edge_p<false, true, true, T, Out> : k_march_edge_p<false, true, false, T, Out>);
+                return;
+            }
         }
+        if (identity) launch(mac.pow2 ? k_march_edge_p<true, false, true, T, Out> : k_march_edge_p<true, false, false, T, Out>);
+        else launch(mac.pow2 ? k_march_edge_p<false, false, true, T, Out> : k_march_edge_p<false, false, false, T, Out>);
     });
 }
 template <class Out>

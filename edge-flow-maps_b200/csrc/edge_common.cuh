@@ -110,13 +110,6 @@ EDGE_D float N2(float x) {
     else if (a < 1.5f) { float t = 1.5f - a; r = 0.5f * (t * t); }
     return r;
 }
-EDGE_D float dN2(float x) {
-    float a = fabsf(x);
-    float r = 0.0f;
-    if (a < 0.5f) r = -2.0f * a;
-    else if (a < 1.5f) r = 0.5f * (2.0f * a - 3.0f);
-    return x < 0.0f ? -r : r;
-}
 
 // One axis of interp_2 / interp_grad_2 (taichi_utils.py:254-319): the clamped
 // grid coordinate, the first of the three taps that carry weight (the 4th tap
@@ -146,8 +139,8 @@ EDGE_D Axis3<GRAD> bspline_axis(float u, float hi_) {
     const float x0 = s - bf;
     a.base = (int)bf;
     // x0 lies in [0.5, 1.5) (exactly: s - bf is exact), so the branches of
-    // N2 / dN2 at x0, x0 - 1 and x0 - 2 are known: the same values as the
-    // general functions, without their compares.  The third tap's zero
+    // N2 and its derivative at x0, x0 - 1 and x0 - 2 are known: the same values
+    // as the general functions', without their compares.  The third tap's zero
     // branch (|x0 - 2| = 1.5, i.e. x0 = 0.5) needs no select either: there
     // t2 = x0 - 0.5 = 0.  Every difference below is exact, so the first and
     // third derivatives (2 |x| - 3) / 2 are x0 - 1.5 and x0 - 0.5.
