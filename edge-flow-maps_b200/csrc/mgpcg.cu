@@ -2045,8 +2045,12 @@ inline int cu(cudaError_t e) { return e == cudaSuccess ? EDGE_OK : (int)e; }
 constexpr int kMaxBlocks = 148 * 8;
 inline int rgrid(long long n) { return (int)std::max<long long>(1, std::min<long long>(grid_for(n), kMaxBlocks)); }
 
-// Four cells of a line per thread where that leaves a wave of threads, two
-// below (a solve of 32^3: 388 us with two, 392 us with four).
+// Four cells of a line per thread on large grids, two on small ones, which want
+// the threads (us of a solve of one iteration, two and four: 32^3 132 and 134,
+// 64x32x32 158 and 163, 64^3 178 and 180, 96^3 266 and 263, 128x128x64 288 and
+// 285, 192x96x96 299 and 292, 256x128x128 444 and 436).  The sizes cross near
+// 3e5 cells, but a sum's order is that of its threads, and with it the last bits
+// of a solve: the line stays where it was drawn.
 template <class F>
 void with_lines(const Lvl& L, F f) {
     const long long n = (long long)L.n0 * L.n1 * L.n2;
