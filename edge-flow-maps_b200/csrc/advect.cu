@@ -1611,6 +1611,15 @@ int edge_march_fields(int variant, int nx, int ny, int nz, float dx, float dt, f
     return launch_status();
 }
 
+int edge_face_map_launches(int nx, int ny, int nz, float dx) {
+    if (!dims_ok(nx, ny, nz)) return EDGE_EINVAL;
+    // with a power-of-two spacing only the last cell centre of an axis can be
+    // off its cell: there the clamp bound n-2-1e-6 may be below n-2 in float32
+    const MapP m = make_mapp(nullptr, nx, ny, nz, dx);
+    auto whole = [](float x) { return x == floorf(x); };
+    return m.pow2 && whole(m.hi[0]) && whole(m.hi[1]) && whole(m.hi[2]) ? 1 : 2;
+}
+
 int edge_face_map_packed(int variant, int nx, int ny, int nz, float dx, const float* packed, float* fpsix,
                          float* fpsiy, float* fpsiz, float* fcolx, float* fcoly, float* fcolz, void* stream) {
     if (!dims_ok(nx, ny, nz) || planes_of(variant) < 0 || !packed || !fpsix || !fpsiy || !fpsiz || !fcolx ||
@@ -1623,10 +1632,7 @@ int edge_face_map_packed(int variant, int nx, int ny, int nz, float dx, const fl
     const int g = grid_for(m.n, 128);
     if (m.pow2) k_face_line_p<true><<<g, 128, 0, st>>>(m, fp, fc);
     else k_face_line_p<false><<<g, 128, 0, st>>>(m, fp, fc);
-    // with a power-of-two spacing only the last cell centre of an axis can be
-    // off its cell: there the clamp bound n-2-1e-6 may be below n-2 in float32
-    auto whole = [](float x) { return x == floorf(x); };
-    if (m.pow2 && whole(m.hi[0]) && whole(m.hi[1]) && whole(m.hi[2])) return launch_status();
+    if (edge_face_map_launches(nx, ny, nz, dx) == 1) return launch_status();
     // 16 blocks per SM where the grid has the faces for it: a block's collected
     // faces take one or two rounds of its threads
     const long long nf = n_faces(nx, ny, nz);

@@ -6,9 +6,7 @@ tensors) unless stated.  Shapes are checked here; the library re-checks sizes
 and pointers.
 """
 import ctypes
-import math
 
-import numpy as np
 import torch
 
 from . import _native as N
@@ -185,9 +183,12 @@ def march_ge_packed(u, dx, dt, packed_in, packed_out, res):
 
 
 def face_map_packed(variant, dx, packed, res, fpsi, fcol):
+    """face_map on a packed map.  A face on the line between two cell centres
+    takes its values from those two cells (the same bits on a finite map): what
+    is not finite in a cell reaches the faces of that cell only, where face_map
+    multiplies it by a weight of zero for its neighbours' faces too."""
     _call("edge_face_map_packed", variant, *res, F(dx), ptr(packed), *_p3(fpsi), *_p3(fcol), stream())
-    # a second launch takes the faces that rounding puts off the line between two cell centres
-    _launched[0] += int(math.frexp(dx)[0] != 0.5 or any(np.float32(n - 2 - 1e-6) != n - 2 for n in res))
+    _launched[0] += N.load().edge_face_map_launches(*res, F(dx)) - 1
 
 
 def face_map(variant, dx, psi, T, dT, d2T, fpsi, fcol):

@@ -168,9 +168,15 @@ int edge_march_fields(int variant, int nx, int ny, int nz, float dx, float dt, f
  * alias in_packed. */
 int edge_march_ge_packed(int nx, int ny, int nz, float dx, float dt, const float *ux, const float *uy,
                          const float *uz, const float *in_packed, float *out_packed, void *stream);
-/* edge_face_map on a packed map */
+/* edge_face_map on a packed map.  A face between two cell centres takes psi and
+ * its derivative from those two cells, the same bits on a finite map; the other
+ * six cells of the full contraction have weights of zero there and are not read,
+ * so that a value of theirs that is not finite does not reach the face (in
+ * edge_face_map it does, as zero times infinity).  edge_face_map_launches: the
+ * kernels it launches, the second for faces that rounding puts off that line. */
 int edge_face_map_packed(int variant, int nx, int ny, int nz, float dx, const float *packed, float *fpsix,
                          float *fpsiy, float *fpsiz, float *fcolx, float *fcoly, float *fcolz, void *stream);
+int edge_face_map_launches(int nx, int ny, int nz, float dx);
 /* forward map on the faces, advance_map x3, run_edge.py:330-357 (in place) */
 int edge_advance_map(int nx, int ny, int nz, float dx, float dt, const float *ux, const float *uy, const float *uz,
                      float *phix, float *phiy, float *phiz, float *Fx, float *Fy, float *Fz, void *stream);
