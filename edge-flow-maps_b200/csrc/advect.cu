@@ -236,8 +236,11 @@ struct FieldsOut {
 // The per-cell accumulators (the centre point's psi and Jacobian, the A and B
 // groups of the mixed derivatives) live in shared memory, one column per
 // thread, so that the registers hold only the current point's trajectory: four
-// blocks of 128 threads per SM (the pairs of hermite3p_pairs spill at five;
-// from the identity, which has no Hermite contraction, five).  Bound by issue
+// blocks of 128 threads per SM, five from the identity, which has no Hermite
+// contraction (us at three, four and five: 64x32x32 62, 60, 64, 256x128x128 2800,
+// 2667, 2690, 192x96x96, whose spacing is no power of two, 1343, 1272, 1236; from
+// the identity at four, five and six 256x128x128 1565, 1591, 1743, 192x96x96 712,
+// 709, 811).  Four spill 60 to 140 bytes, five about as much.  Bound by issue
 // slots and FP32 register ports.  256x128x128: 3387 -> 2650 us, 64x32x32 76 ->
 // 61 us, from the identity 2026 -> 1600 us, with samples from the block's tile
 // and paired contractions.
