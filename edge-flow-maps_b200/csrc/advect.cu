@@ -852,8 +852,11 @@ __global__ void __launch_bounds__(128) k_face_map(MapF m, float* fpx, float* fpy
     }
 }
 
-// advance_map x3 (run_edge.py:330-357).  Six blocks per SM: 256x128x128 1118 us
-// uncapped, 1090 at six, 1133 at eight.
+// advance_map x3 (run_edge.py:330-357).  Bound by issue (70 %) and, as the map
+// ages and a warp's points part, by gathers.  us uncapped, at six blocks per SM
+// and at eight, for a map just reset and for one of eleven steps at half a cell:
+// 192x96x96 501, 458, 495 and 669, 655, 800; 256x128x128, whose spacing needs no
+// divisions, 979, 992, 1023 and 1267, 1290, 1355.
 template <bool P2>
 __global__ void __launch_bounds__(128, 6) k_advance_map(Mac mac_, float dt, float* phix, float* phiy, float* phiz,
                                                      float* Fx, float* Fy, float* Fz) {
@@ -981,9 +984,10 @@ __global__ void __launch_bounds__(T::threads) k_advect_tile(Mac mac_, float dt, 
 }
 
 // map_u / map_u_psi pullback with fused BFECC arithmetic (edge_pullback_u).
-// Waits for its gathers, so more warps are worth a few spills: 256x128x128
-// 318 us uncapped, 287 at six blocks per SM; with the divisions of a spacing
-// that is no power of two five (192x96x96 127 and 126 us, 130 at six).
+// Waits for its gathers, so more warps are worth a few spills: through a map
+// just reset and one of eleven steps, 256x128x128 334 and 387 us uncapped, 299
+// and 371 at six blocks per SM; with the divisions of a spacing that is no power
+// of two five (192x96x96 141 and 139 us, six was slower).
 template <bool P2>
 __global__ void __launch_bounds__(256, P2 ? 6 : 5) k_pullback_u(Mac mac_, Face3 pos, Face3 col, Face3 init, float scale, Face3 sub,
                                                     float* ox, float* oy, float* oz) {
