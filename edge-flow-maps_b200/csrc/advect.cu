@@ -1304,8 +1304,9 @@ inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 // 330 and 325; 80x48x40 92 and 91, 177 and 149).  A warp with a sample outside
 // its tile reads global memory, from four rows of eight cells instead of one of
 // 32, so steps of four cells and more, which no driver takes, cost more than
-// without tiles where rows are whole lines: 64x32x32 at four cells EDGE 80 and
-// 73, ED8 111 and 98, 64^3 EDGE 203 and 205, ED8 267 and 259.
+// without tiles where rows are whole lines: at four cells 64x32x32 EDGE 80 us
+// and 73, ED8 111 and 98, 128x32x32 EDGE 141 and 121, ED8 209 and 168, 64^3 EDGE
+// 203 and 205, ED8 267 and 259.
 using CellTile = Tile<4, 4, 8>;
 template <class F>
 void with_tile(int nx, int ny, int nz, double fill, F f) {
