@@ -28,13 +28,20 @@ def test_accumulated_map_of_another_size_is_refused(at, other):
 
 # the packed copy of the map is float32 whatever torch's default type is
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float16, torch.bfloat16, torch.float32])
-def test_scratch_under_another_default_dtype(dtype):
+def test_scratch_under_another_default_dtype(dtype, monkeypatch):
     from edgeb200 import ops
+    res = (4, 5, 6)
+    u = [torch.zeros(s) for s in ((5, 5, 6), (4, 6, 6), (4, 5, 7))]
+    m, o = _fields(res, 7), _fields(res, 7)
+    seen, empty = [], torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: seen.append(empty(*a, **k)) or seen[-1])
     before = torch.get_default_dtype()
-    psi = torch.zeros((4, 5, 6, 3), dtype=torch.float32)
     torch.set_default_dtype(dtype)
     try:
-        work = ops._map_workspace(psi)
+        with pytest.raises(ValueError, match="CUDA"):  # tensors of the host go no further
+            ops.march_edge(u, 0.25, 0.01, 0.01, m[0], m[1:4], m[4:], o[0], o[1:4], o[4:])
+        with pytest.raises(ValueError, match="CUDA"):
+            ops.march_ed4(u, 0.25, 0.01, 0.01, m[0], m[1:4], o[0], o[1:4])
     finally:
         torch.set_default_dtype(before)
-    assert work.dtype == torch.float32 and work.numel() == 8 * 4 * 4 * 5 * 6
+    assert [(t.dtype, t.numel()) for t in seen] == [(torch.float32, 8 * 4 * 4 * 5 * 6)] * 2
