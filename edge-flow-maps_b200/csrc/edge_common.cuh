@@ -196,9 +196,6 @@ struct VRows {
         return (o & 2) ? VRow{{s2, s3, s4}} : VRow{{s0, s1, s2}};
     }
 };
-// whether the rows of a sample whose first tap is (x, y, .) have another row of
-// the field before and after them, so that no wide load passes its ends
-EDGE_D bool rows_inside(int x, int y, int n0, int n1) { return (x > 0 || y > 0) && (x + 3 < n0 || y + 3 < n1); }
 template <bool WIDE>
 EDGE_D VRows<WIDE> vrows(const float* f, int x, int y, int z, int n1, int n2) {
     return VRows<WIDE>{f + (((long long)x * n1 + y) * n2 + z), n1, n2};
@@ -339,26 +336,28 @@ EDGE_D void mac_sums(const Mac& m, const Axis3<GRAD> A0[3], const Axis3<GRAD> A5
 // wavefronts than three scalar ones.  So a warp takes wide loads where more than
 // kPointGroups of its points lie apart from the one before.  us, always wide,
 // always scalar and so: 10^6 points at random in 128x256x128 135, 164, 131; in
-// a ball 115, 148, 113; on a lattice 88, 31, 37; sorted by cell 85, 48, 51; in
-// runs of two 89, 87, 78, of four 90, 52, 55.
+// a ball 113, 148, 111; on a lattice 92, 31, 35; sorted by cell 88, 49, 51; in
+// runs of two 92, 87, 76, of four 88, 52, 53.
 constexpr int kPointGroups = 10;
 EDGE_D void mac_sample_points(const Mac& m, const float p[3], unsigned mask, float v[3]) {
     float q[3];
     Axis3<false> A0[3], A5[3];
     mac_axes<false>(m, p, q, A0, A5);
     const int x0 = A0[0].base, y0 = A0[1].base, z0 = A0[2].base, x5 = A5[0].base, y5 = A5[1].base, z5 = A5[2].base;
-    const int xy = (x0 << 16) ^ y0, bxy = __shfl_up_sync(mask, xy, 1), bz = __shfl_up_sync(mask, z0, 1);
-    const bool apart = abs((xy >> 16) - (bxy >> 16)) > 1 || abs((xy & 0xffff) - (bxy & 0xffff)) > 1 || abs(z0 - bz) > 16;
-    const bool inside = rows_inside(x0, y5, m.nx + 1, m.ny) && rows_inside(x5, y0, m.nx, m.ny + 1) &&
-                        rows_inside(x5, y5, m.nx, m.ny);
+    // apart: not within a cell or so in x and y of the lane before
+    const unsigned xy = ((unsigned)x0 << 16) + (unsigned)y0, step = xy - __shfl_up_sync(mask, xy, 1) + 0x00010001u;
+    const bool apart = (step & 0xfffcfffcu) != 0;
     auto sums = [&](auto wide) {
         constexpr bool W = decltype(wide)::value;
         v[0] = bspline_rows(vrows<W>(m.u[0], x0, y5, z5, m.ny, m.nz), A0[0], A5[1], A5[2]);
         v[1] = bspline_rows(vrows<W>(m.u[1], x5, y0, z5, m.ny + 1, m.nz), A5[0], A0[1], A5[2]);
         v[2] = bspline_rows(vrows<W>(m.u[2], x5, y5, z0, m.ny, m.nz + 1), A5[0], A5[1], A0[2]);
     };
-    if (__popc(__ballot_sync(mask, apart)) > kPointGroups && __all_sync(mask, inside)) sums(std::true_type{});
-    else sums(std::false_type{});
+    if (__popc(__ballot_sync(mask, apart)) > kPointGroups &&
+        __all_sync(mask, (x5 > 0 || y5 > 0) && (x0 + 3 < m.nx || y0 + 3 < m.ny)))
+        sums(std::true_type{});
+    else
+        sums(std::false_type{});
 }
 // the lanes of a warp (of a one-dimensional block) whose index is below n, for
 // a thread e that is one of them
